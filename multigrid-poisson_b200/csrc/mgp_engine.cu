@@ -33,6 +33,7 @@
 #include "mgp_kernels.cuh"
 #include "mgp_wave.cuh"
 #include "mgp_tail.cuh"
+#include "mgp_cluster.cuh"
 
 using namespace mgp;
 
@@ -1180,12 +1181,266 @@ int launch_tail(mgp_solver* s, int t0, bool fcycle, double omega, int64_t ns) {
     return launch_k(s, k_tail<T>, dim3(1), dim3(kTailThreads), smem, a);
 }
 
+// ---- the coarse levels in one cluster (mgp_cluster.cuh) -----------------------------------
+constexpr size_t kClMaxSmem = 216 * 1024;  // dynamic; the argument copy and reduction slots fit beside it
+
+// CTAs of the largest cluster this device co-schedules with that much shared memory: 16 (opt-in
+// size), 8, or 0 (none).
+int cluster_ctas(int dev) {
+    static std::mutex mu;
+    static int cached[64] = {};  // 0: not asked yet, else CTAs + 1
+    std::lock_guard<std::mutex> lk(mu);
+    int& c = cached[dev & 63];
+    if (c) return c - 1;
+    int best = 0;
+    auto kernels = {(const void*)k_cluster<double, true>, (const void*)k_cluster<double, false>,
+                    (const void*)k_cluster<float, true>, (const void*)k_cluster<float, false>};
+    for (int n : {16, 8}) {
+        bool ok = true;
+        for (const void* k : kernels) {
+            cudaLaunchAttribute attr[1];
+            attr[0].id = cudaLaunchAttributeClusterDimension;
+            attr[0].val.clusterDim.x = n;
+            attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+            cudaLaunchConfig_t cfg = {};
+            cfg.gridDim = dim3(n);
+            cfg.blockDim = dim3(kClMaxThreads);
+            cfg.dynamicSmemBytes = kClMaxSmem;
+            cfg.attrs = attr;
+            cfg.numAttrs = 1;
+            int active = 0;
+            ok = ok && cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kClMaxSmem) == cudaSuccess &&
+                 cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
+                 cudaOccupancyMaxActiveClusters(&active, k, &cfg) == cudaSuccess && active >= 1;
+        }
+        if (ok) {
+            best = n;
+            break;
+        }
+    }
+    cudaGetLastError();  // a refused size leaves an error behind
+    c = best + 1;
+    return best;
+}
+
+unsigned div_magic(int d) { return d <= 1 ? 0u : (unsigned)(((1ull << 32) + d - 1) / d); }
+
+// Planes of a CTA's slab: at least two in every slab, the last one included (the east and west
+// face restriction reads three planes from the face inwards, two slabs' worth at most).
+int slab_planes(int nx, int nc) {
+    int P = std::max(2, (nx + nc - 1) / nc);
+    while (P < nx && nx % P == 1) P++;
+    return std::min(P, nx);
+}
+
+// Slab shape and shared-memory offsets of levels t..L-1 in a cluster of `nc` CTAs; false when
+// they do not fit.  `lev` (may be null) receives them, *smem / *threads the launch's.
+template <typename T>
+bool cluster_plan(const mgp_solver* s, int t, int nc, ClArgs<T>* a, size_t* smem, int* threads) {
+    const bool jac = s->desc.relaxation == MGP_JACOBI;
+    long long off = 0, gather = 0;
+    int nt = 256;
+    for (int m = t; m < s->levels; m++) {
+        const LevelState& L = s->lv[m];
+        const Geom& G = L.G;
+        const int P = slab_planes(G.nx, nc);
+        const long long pl = (long long)G.ny * G.nz;
+        if (pl * (4 * P + 6) * (long long)sizeof(T) > (long long)kClMaxSmem * 2) return false;
+        const int ncol = std::max(0, G.y1 - G.y0) * std::max(0, G.z1 - G.z0);
+        const int nitem = jac ? ncol : std::max(0, G.y1 - G.y0) * ((std::max(0, G.z1 - G.z0) + 1) / 2);
+        // Threads: one per relaxation item of the finest level, or even passes over the items; an
+        // operation's set-up per warp counts, so no more than that (at least 8 warps: the Neumann
+        // faces are dealt out to warps).
+        if (m == t) {
+            const int passes = std::max(1, (nitem + kClMaxThreads - 1) / kClMaxThreads);
+            nt = std::max(256, ((nitem + passes - 1) / passes + 31) / 32 * 32);
+        }
+        auto split = [&](int n) { return n ? std::max(1, std::min(P, nt / n)) : 1; };
+        const int nseg = split(nitem), rseg = split(ncol);
+        ClLevel<T> q{};
+        q.G = G;
+        q.P = P;
+        q.nact = (G.nx + P - 1) / P;
+        q.pl = (int)pl;
+        q.nseg = nseg;
+        q.seglen = (P + nseg - 1) / nseg;
+        q.m_nz = div_magic(G.nz);
+        q.m_ny = div_magic(G.ny);
+        q.m_pl = div_magic((int)pl);
+        q.m_P = div_magic(P);
+        q.ncol = ncol;
+        q.m_col = div_magic(ncol);
+        q.nitem = nitem;
+        q.m_item = div_magic(nitem);
+        q.rseg = rseg;
+        q.rlen = (P + rseg - 1) / rseg;
+        auto take = [&](long long n) {
+            const long long o = off;
+            off += n;
+            return (int)o;
+        };
+        q.so_u[0] = take((P + 2) * pl);
+        q.so_u[1] = jac ? take((P + 2) * pl) : q.so_u[0];
+        q.so_f = take(P * pl);
+        q.so_r = take((P + 2) * pl);
+        for (int f = 0; f < 6; f++) {
+            q.neumann[f] = s->face_kind[f] == MGP_NEUMANN;
+            const long long n = f == MGP_EAST || f == MGP_WEST ? pl : (long long)(P + 2) * (f <= MGP_SOUTH ? G.nz : G.ny);
+            q.so_g[f] = q.neumann[f] ? take(n) : 0;
+        }
+        if (m > t) {
+            const LevelState& F = s->lv[m - 1];
+            const int Pf = slab_planes(F.G.nx, nc);
+            gather = std::max(gather, ((Pf + 2) / 2 + 3) * pl);
+        }
+        if (off * (long long)sizeof(T) > (long long)kClMaxSmem) return false;
+        if (a) a->L[m - t] = q;
+    }
+    if (a) a->so_gather = (int)off;
+    off += gather;
+    long long bytes = off * (long long)sizeof(T);
+    for (int m = t; m < s->levels; m++) {  // the column tables
+        const Geom& G = s->lv[m].G;
+        const int wy = std::max(0, G.y1 - G.y0), wz = std::max(0, G.z1 - G.z0);
+        if (a) {
+            a->L[m - t].so_tab = (int)bytes;
+            a->L[m - t].so_pair = (int)bytes + 4 * wy * wz;
+        }
+        bytes += 4ll * wy * (wz + (jac ? 0 : (wz + 1) / 2));
+    }
+    *smem = (size_t)bytes;
+    *threads = nt;
+    return *smem <= kClMaxSmem;
+}
+
+// First level of the cluster's visits (s->levels: none): the finest level whose hierarchy fits in
+// one cluster's shared memory (about 36K points in FP64).  An operation takes 0.8-1.7 us there
+// against 2.5-3 us as a launch of its own; ten 65^3 red-black F-cycles 3.42 -> 2.56 ms, four FP32
+// 257^3 F-cycles 5.08 -> 4.20 ms, four 33x17x17 F-cycles with their set-up 0.488 -> 0.375 ms.  Not
+// for column-ordered Gauss-Seidel (its sweep runs along x),
+// levels with wavefront buffers, or levels whose launch shapes or set-up form were asked for
+// (they are shapes of the per-level kernels), nor beside the one-CTA form.
+int cluster_level(const mgp_solver* s) {
+    if (s->levels < 2 || s->pool || (s->desc.flags & MGP_FLAG_FUSED_SETUP) || s->lv[0].tune[MGP_TUNE_TAIL]) return s->levels;
+    const int nc = cluster_ctas(s->device);
+    if (!nc) return s->levels;
+    for (int l = std::max(0, s->levels - kClMaxLevels); l < s->levels - 1; l++) {
+        bool ok = true;
+        for (int m = l; m < s->levels && ok; m++) {
+            ok = !s->lv[m].gs_column && !s->lv[m].pair;
+            for (int p = 0; p < MGP_TUNE_PARAMS; p++) ok = ok && !s->lv[m].tune[p];
+        }
+        size_t smem = 0;
+        int threads = 0;
+        if (ok && (s->dtype == MGP_F64 ? cluster_plan<double>(s, l, nc, nullptr, &smem, &threads)
+                                       : cluster_plan<float>(s, l, nc, nullptr, &smem, &threads)))
+            return l;
+    }
+    return s->levels;
+}
+
+// One visit of levels t..L-1: F(t) when `f`, then V(t) when `v`, then (level 0 only) the solve
+// loop's residual with its max-norm into *norm when `norm`.
+template <typename T>
+int launch_cluster(mgp_solver* s, int t, bool f, bool v, double omega, int64_t ns, unsigned long long* norm = nullptr) {
+    static_assert(sizeof(ClArgs<T>) % sizeof(int) == 0, "the kernel copies its arguments as ints");
+    ClArgs<T> a{};
+    size_t smem = 0;
+    int threads = 0;
+    const int nc = cluster_ctas(s->device);
+    if (!cluster_plan<T>(s, t, nc, &a, &smem, &threads)) return fail(MGP_ERR_STATE, "coarse levels do not fit a cluster");
+    const bool jac = s->desc.relaxation == MGP_JACOBI;
+    a.nl = s->levels - t;
+    a.ns = (int)ns;
+    a.fw = s->desc.restriction == MGP_FULLWEIGHTING;
+    a.alt = s->gs_alternate;
+    a.norm = norm;
+    a.err = s->err_word;
+    for (int m = 0; m < a.nl; m++) {
+        LevelState& L = s->lv[t + m];
+        ClLevel<T>& q = a.L[m];
+        q.ub[0] = (T*)L.ubuf[0];
+        q.ub[1] = jac ? (T*)L.ubuf[1] : nullptr;
+        q.f = (T*)L.f;
+        q.r = (T*)L.r;
+        for (int c = 0; c < 6; c++) q.g[c] = (T*)L.face[c];
+        // constants as launch_stencil and bc_args form them: omega is rounded to T first
+        const T om = (T)omega;
+        q.two_h = (T)(2.0 * L.h);
+        q.hsq = (T)(L.h * L.h);
+        q.one_omega = (T)(1.0 - om);
+        q.omega_sixth = (T)(om / 6.0);
+        q.h = (T)L.h;
+        hsq_terms(q.hsq, q.inv_hsq, q.pow2);
+        a.cur |= (unsigned)(L.cur & 1) << m;
+    }
+    auto emit = [&](int op, int m) {
+        if (a.nops < kClMaxOps) {
+            a.op[a.nops] = (unsigned char)op;
+            a.lv[a.nops] = (unsigned char)m;
+        }
+        a.nops++;
+    };
+    // the recursion of vcycle_t / fcycle_t, and the host state it leaves (each Jacobi sweep swaps
+    // the pair; red-black relaxations flip `alternate` an even number of times)
+    bool skip = s->lv[t].first_done;
+    auto relax = [&](int m) {
+        emit(skip ? CL_RELAX_SKIP1 : CL_RELAX, m);
+        skip = false;
+        if (jac) s->lv[t + m].cur ^= (int)(ns & 1);
+    };
+    std::function<void(int)> vc = [&](int m) {
+        relax(m);
+        if (m >= a.nl - 1) return;
+        emit(CL_SETUP, m);
+        vc(m + 1);
+        emit(CL_PROLONG, m);
+        relax(m);
+    };
+    std::function<void(int)> fc = [&](int m) {
+        relax(m);
+        emit(CL_SETUP, m);
+        if (m + 1 < a.nl - 1) fc(m + 1);
+        vc(m + 1);
+        emit(CL_PROLONG, m);
+    };
+    const uint64_t before = state_bits(s);
+    if (f) fc(0);
+    if (v) vc(0);
+    if (norm) emit(CL_NORM, 0);
+    if (a.nops > kClMaxOps) {
+        set_state_bits(s, before);
+        return fail(MGP_ERR_STATE, "coarse-level visit of %d operations", a.nops);
+    }
+    for (int m = 0; m < a.nl; m++) s->lv[t + m].first_done = false;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = nc;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(nc);
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s->stream;
+    cfg.attrs = attr;
+    cfg.numAttrs = pdl_enabled() ? 2 : 1;
+    const cudaError_t e = jac ? cudaLaunchKernelEx(&cfg, k_cluster<T, true>, a) : cudaLaunchKernelEx(&cfg, k_cluster<T, false>, a);
+    if (e != cudaSuccess) return fail(MGP_ERR_CUDA, "kernel launch: %s", cudaGetErrorString(e));
+    return check_launch(s);
+}
+
 // tail_norm: the caller's residual of level l with its max-norm, right after this cycle (the
 // solve loop's); the cycle's last relaxation may take it over and then sets *tail_done.
 template <typename T>
 int vcycle_t(mgp_solver* s, int l, double omega, int64_t ns, unsigned long long* tail_norm = nullptr,
              bool* tail_done = nullptr) {
     // Vcycle<T> (include/vcycle.h:14-98)
+    if (ns >= 1 && l >= cluster_level(s)) {
+        if (tail_done) *tail_done = tail_norm != nullptr;
+        return launch_cluster<T>(s, l, false, true, omega, ns, tail_norm);
+    }
     if (!tail_norm && l >= 1 && l == tail_level(s)) return launch_tail<T>(s, l, false, omega, ns);
     const int tail = tail_norm ? RESID_NORM : RESID_NONE;
     if (l >= s->levels - 1) return relax_t<T>(s, l, omega, ns, false, tail, tail_norm, tail_done);
@@ -1208,13 +1463,22 @@ int fcycle_t(mgp_solver* s, int l, double omega, int64_t ns, unsigned long long*
              bool* tail_done = nullptr) {
     // Fcycle<T> (include/fcycle.h:13-97); the V-cycle of this level that follows relaxes it again
     if (tail_done) *tail_done = false;
+    const int cl = ns >= 1 ? cluster_level(s) : s->levels;
+    if (l >= cl) {
+        if (tail_done) *tail_done = tail_norm != nullptr;
+        return launch_cluster<T>(s, l, true, l == 0, omega, ns, tail_norm);
+    }
     if (!tail_norm && l >= 1 && l == tail_level(s)) return launch_tail<T>(s, l, true, omega, ns);
     bool rd = false;
     CKS(relax_t<T>(s, l, omega, ns, /*later=*/true, setup_residual_separate(s, l) ? RESID_STORE : RESID_NONE, nullptr,
                    &rd));
     CKS(coarse_setup_t<T>(s, l, omega, ns, rd));
-    if (l < s->levels - 2) CKS(fcycle_t<T>(s, l + 1, omega, ns));
-    CKS(vcycle_t<T>(s, l + 1, omega, ns));
+    if (l + 1 >= cl) {  // F(l+1) and V(l+1) in one launch
+        CKS(launch_cluster<T>(s, l + 1, l < s->levels - 2, true, omega, ns));
+    } else {
+        if (l < s->levels - 2) CKS(fcycle_t<T>(s, l + 1, omega, ns));
+        CKS(vcycle_t<T>(s, l + 1, omega, ns));
+    }
     CKS((prolong_t<T, true>(s, l)));
     if (l == 0) CKS(vcycle_t<T>(s, 0, omega, ns, tail_norm, tail_done));
     return MGP_OK;
