@@ -75,9 +75,9 @@ struct TUpdate {
 };
 template <typename Ti>
 struct TRefRes {
-    using Args = RefineArgs<double, Ti>;
+    using Args = RefineArgs<double, Ti, false>;
     static __device__ __forceinline__ void run(const Args& a, int bx, int by, int) {
-        refine_residual_tile<double, Ti, false>(a, bx, by);
+        stencil_tile<double, OP_RESIDUAL, true, false, Args>(a, bx, by);
     }
 };
 
@@ -365,7 +365,7 @@ int build_step(mgp_batch* b, ScheduleBuilder& sb) {
     // u += e, then the new FP64 residual, its right-hand side for the next correction and the
     // per-problem norm
     std::vector<BatchItem<UpdateArgs<double, Ti>>> ups;
-    std::vector<BatchItem<RefineArgs<double, Ti>>> rrs;
+    std::vector<BatchItem<RefineArgs<double, Ti, false>>> rrs;
     double act_points = 0.0;
     for (auto* p : act) {
         const Geom& G = p->s->lv[0].G;
@@ -379,20 +379,7 @@ int build_step(mgp_batch* b, ScheduleBuilder& sb) {
         UpdateArgs<double, Ti> ua{(double*)u_ptr(s, 0), L.G, (const Ti*)u_ptr(in, 0), I.G.sx, I.G.sy};
         constexpr int Vd = VecT<double>::V;
         push_item(ups, ua, (L.G.ny * ((L.G.nz + Vd - 1) / Vd) + kThreads - 1) / kThreads, L.G.nx);
-        RefineArgs<double, Ti> ra;
-        ra.G = L.G;
-        ra.u = (const double*)u_ptr(s, 0);
-        ra.f = (const double*)L.f;
-        ra.r = (double*)L.r;
-        ra.F = faces_of<double>(s, 0);
-        ra.two_h = 2.0 * L.h;
-        ra.hsq = L.h * L.h;
-        hsq_terms(ra.hsq, ra.inv_hsq, ra.hsq_pow2);
-        ra.sxi = I.G.sx;
-        ra.syi = I.G.sy;
-        ra.fi = (Ti*)I.f;
-        ra.ui = (Ti*)u_ptr(in, 0);
-        ra.norm = b->d_norms + p->slot;
+        auto ra = refine_args<Ti, false>(s, RefineFirst{}, b->d_norms + p->slot);
         constexpr int V = VecT<double>::V;
         const int plane = L.G.ny * ((L.G.nz + V - 1) / V);
         const int bx = (plane + kThreads - 1) / kThreads;
@@ -503,7 +490,7 @@ int batch_start_new(mgp_batch* b) {
         if (st == MGP_OK && e == cudaSuccess) e = cudaStreamSynchronize(s->stream);
         if (st == MGP_OK && e == cudaSuccess) {
             memcpy(&p.fnorm, b->h_norms + p.slot, 8);
-            st = refine_residual(s, false);  // zeroes the inner guess, norm into the slot
+            st = refine_residual(s);  // zeroes the inner guess, norm into the slot
         }
         if (st == MGP_OK && e == cudaSuccess) e = cudaMemcpyAsync(b->h_norms + p.slot, s->d_norm, 8, cudaMemcpyDeviceToHost, s->stream);
         if (st == MGP_OK && e == cudaSuccess) e = cudaStreamSynchronize(s->stream);
@@ -765,7 +752,7 @@ int mgp_batch_solve(mgp_batch* b, double tol, int64_t maxiter, int64_t* steps) {
     for (auto& p : b->probs)
         if (p.s) {
             std::swap(p.s->stream, b->stream);
-            int st = refine_residual(p.s, true);
+            int st = refine_store_residual(p.s);
             std::swap(p.s->stream, b->stream);
             CKS(st);
         }

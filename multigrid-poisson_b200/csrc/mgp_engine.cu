@@ -1557,35 +1557,65 @@ int read_norm(mgp_solver* s, double* out) {
 }
 
 // ---- iterative refinement ------------------------------------------------------------
-template <typename Ti>
-int refine_residual_t(mgp_solver* s, bool write_r) {
+// The inner first sweep that the refinement residual writes along (RefineArgs::first): the
+// smoothing of the correction cycle that follows.
+struct RefineFirst {
+    int on = 0;  // 0 none, 1 Jacobi, 2 red-black
+    double omega = 0;
+};
+RefineFirst refine_first(const mgp_solver* in, double omega, int64_t ns) {
+    RefineFirst w;
+    if (ns >= 1 && !in->lv[0].gs_column && !in->lv[0].wave) w.on = in->desc.relaxation == MGP_JACOBI ? 1 : 2;
+    w.omega = omega;
+    return w;
+}
+
+// Arguments and grid of one refinement residual; chunks as the caller cuts them.
+template <typename Ti, bool R>
+RefineArgs<double, Ti, R> refine_args(mgp_solver* s, const RefineFirst& w, unsigned long long* norm) {
     mgp_solver* in = s->inner;
     LevelState& L = s->lv[0];
     LevelState& I = in->lv[0];
-    RefineArgs<double, Ti> a;
+    RefineArgs<double, Ti, R> a{};
     a.G = L.G;
-    a.u = (const double*)u_ptr(s, 0);
+    a.G.poff = I.G.poff;
+    a.src = (const double*)u_ptr(s, 0);
     a.f = (const double*)L.f;
-    a.r = (double*)L.r;
+    a.dst = (double*)L.r;
     a.F = faces_of<double>(s, 0);
     a.two_h = 2.0 * L.h;
     a.hsq = L.h * L.h;
     hsq_terms(a.hsq, a.inv_hsq, a.hsq_pow2);
+    a.norm = norm;
     a.sxi = I.G.sx;
     a.syi = I.G.sy;
     a.fi = (Ti*)I.f;
     a.ui = (Ti*)u_ptr(in, 0);
-    a.norm = s->d_norm;
+    a.uw = (Ti*)uprev_ptr(in, 0);
+    a.first = w.on;
+    a.fcolour = in->gs_alternate ? 0 : 1;
+    const Ti om = (Ti)w.omega;  // the relaxation takes omega as a Ti (jacobi.h:41-44)
+    a.w0 = (Ti)(1.0 - om);
+    a.w1 = (Ti)(om / 6.0);
+    a.hsqi = (Ti)(I.h * I.h);
+    return a;
+}
+
+template <typename Ti, bool R>
+int refine_residual_t(mgp_solver* s, const RefineFirst& w) {
+    LevelState& L = s->lv[0];
+    auto a = refine_args<Ti, R>(s, w, s->d_norm);
     constexpr int V = VecT<double>::V;
     const int plane = L.G.ny * ((L.G.nz + V - 1) / V);
     const int bx = (plane + kThreads - 1) / kThreads;
-    const int target = sm_count(s->device) * 8;
-    int chunks = std::max(1, std::min((target + bx - 1) / bx, L.G.nx));
+    const int cap = sm_count(s->device) * resident_blocks(k_refine_residual<double, Ti, R>);
+    int chunks = short_march_chunks<double>(L.G, bx, cap, march_chunks(bx, L.G.nx, cap));
     a.ichunk = (L.G.nx + chunks - 1) / chunks;
     chunks = (L.G.nx + a.ichunk - 1) / a.ichunk;
     CK(cudaMemsetAsync(s->d_norm, 0, sizeof(unsigned long long), s->stream));
-    if (write_r) return launch_k(s, k_refine_residual<double, Ti, true>, dim3(bx, chunks), dim3(kThreads), 0, a);
-    return launch_k(s, k_refine_residual<double, Ti, false>, dim3(bx, chunks), dim3(kThreads), 0, a);
+    CKS(launch_k(s, k_refine_residual<double, Ti, R>, dim3(bx, chunks), dim3(kThreads), 0, a));
+    if (!R) s->inner->lv[0].first_done = w.on != 0;
+    return MGP_OK;
 }
 
 template <typename Ti>
@@ -1599,8 +1629,14 @@ int refine_update_t(mgp_solver* s) {
     return launch_k(s, k_refine_update<double, Ti>, dim3(bx, L.G.nx), dim3(kThreads), 0, a);
 }
 
-int refine_residual(mgp_solver* s, bool write_r) {
-    return s->inner->dtype == MGP_F32 ? refine_residual_t<float>(s, write_r) : refine_residual_t<double>(s, write_r);
+// The FP64 residual and its norm, starting the next correction.
+int refine_residual(mgp_solver* s, const RefineFirst& w = RefineFirst{}) {
+    return s->inner->dtype == MGP_F32 ? refine_residual_t<float, false>(s, w) : refine_residual_t<double, false>(s, w);
+}
+// The FP64 residual stored in r (the user-visible residual), and its norm.
+int refine_store_residual(mgp_solver* s) {
+    const RefineFirst w;
+    return s->inner->dtype == MGP_F32 ? refine_residual_t<float, true>(s, w) : refine_residual_t<double, true>(s, w);
 }
 
 // One refinement step, captured once per (cycle, nsmooth, omega, inner state): the
@@ -1614,6 +1650,8 @@ int launch_refine_step(mgp_solver* s, int cycle, int64_t ns, double omega) {
     if (it == s->graphs.end()) {
         const uint64_t pre = state_bits(in);
         const int64_t s0 = s->launches, i0 = in->launches;
+        const RefineFirst w = refine_first(in, omega, ns);
+        in->lv[0].first_done = w.on != 0;  // the residual before this step wrote the first sweep
         cudaGraph_t g = nullptr;
         CK(cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal));
         int st;
@@ -1624,7 +1662,8 @@ int launch_refine_step(mgp_solver* s, int cycle, int64_t ns, double omega) {
             st = cycle == MGP_CYCLE_V ? vcycle_t<double>(in, 0, omega, ns) : fcycle_t<double>(in, 0, omega, ns);
             if (st == MGP_OK) st = refine_update_t<double>(s);
         }
-        if (st == MGP_OK) st = refine_residual(s, false);
+        if (st == MGP_OK) st = refine_residual(s, w);
+        in->lv[0].first_done = false;
         cudaError_t e = cudaStreamEndCapture(s->stream, &g);
         GraphEntry ge;
         ge.post_state = state_bits(in);
@@ -2608,7 +2647,8 @@ static int solve_refined(mgp_solver* s, int cycle, int64_t ns, double omega, dou
     CK(cudaMemsetAsync(s->d_norm, 0, sizeof(unsigned long long), s->stream));
     CKS(norm_t<double>(s, s->lv[0].f, 0, s->d_norm));
     CKS(read_norm(s, &fnorm));
-    CKS(refine_residual(s, false));
+    CKS(refine_residual(s, refine_first(s->inner, omega, ns)));
+    s->inner->lv[0].first_done = false;  // consumed by the steps' graphs
     CKS(read_norm(s, &rnorm));
     double rel = rnorm / fnorm;
     const double first = rel;
@@ -2627,7 +2667,7 @@ static int solve_refined(mgp_solver* s, int cycle, int64_t ns, double omega, dou
         if (flags & MGP_SOLVE_VERBOSE)
             std::cout << std::setw(4) << it << ": Relative residual: " << std::setw(8) << rel << std::endl;
     }
-    CKS(refine_residual(s, true));  // the user-visible FP64 residual of the returned u
+    CKS(refine_store_residual(s));  // the user-visible FP64 residual of the returned u
     CK(cudaStreamSynchronize(s->stream));
     if (out) {
         out->rel_res = rel;

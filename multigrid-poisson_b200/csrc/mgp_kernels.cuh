@@ -87,24 +87,6 @@ __device__ __forceinline__ void block_max_to(unsigned long long v, unsigned long
 // Stencil ops.
 enum StencilOp { OP_JACOBI = 0, OP_GS = 1, OP_GS_COLUMN = 2, OP_RESIDUAL = 3 };
 
-template <typename T>
-struct StencilArgs {
-    Geom G;
-    const T* src;  // u (or u_prev for Jacobi)
-    T* dst;        // u for Jacobi/GS, r for the residual
-    const T* f;
-    Faces<T> F;
-    T two_h;       // 2*h of this level (T, as the reference's two_h)
-    T hsq;         // h*h (T)
-    T one_omega;   // 1-omega (T)
-    T omega_sixth; // omega/6 (T)
-    T inv_hsq;     // 1/hsq, used only when hsq is a power of two (exact)
-    int hsq_pow2;
-    int colour;    // GS colour (0 red: idx%2==0, 1 black)
-    int ichunk;    // planes per block
-    unsigned long long* norm;  // residual: max |r| over the whole shape (nullptr: none)
-};
-
 // Residual with the reference's promotions: f - (sum - 6.0*u)/hsq (include/residual.h:70-72);
 // T=float evaluates in double because of the double literal 6.0.
 template <typename T>
@@ -185,6 +167,33 @@ __device__ __forceinline__ void stv(double* p, const double (&d)[2]) {
 __device__ __forceinline__ void stv(float* p, const float (&d)[4]) {
     *reinterpret_cast<float4*>(p) = make_float4(d[0], d[1], d[2], d[3]);
 }
+
+template <typename T>
+struct StencilArgs {
+    Geom G;
+    const T* src;  // u (or u_prev for Jacobi)
+    T* dst;        // u for Jacobi/GS, r for the residual
+    const T* f;
+    Faces<T> F;
+    T two_h;       // 2*h of this level (T, as the reference's two_h)
+    T hsq;         // h*h (T)
+    T one_omega;   // 1-omega (T)
+    T omega_sixth; // omega/6 (T)
+    T inv_hsq;     // 1/hsq, used only when hsq is a power of two (exact)
+    int hsq_pow2;
+    int colour;    // GS colour (0 red: idx%2==0, 1 black)
+    int ichunk;    // planes per block
+    unsigned long long* norm;  // residual: max |r| over the whole shape (nullptr: none)
+
+    static constexpr bool kStored = true;  // dst's values outside the relaxation bounds count in the norm
+    static constexpr int V = VecT<T>::V;
+    __device__ __forceinline__ void put(long long p, int, int, int, const T (&v)[V]) const { stv(dst + p, v); }
+    __device__ __forceinline__ void put(long long p, int, int, int, const T (&v)[V], unsigned act) const {
+#pragma unroll
+        for (int e = 0; e < V; e++)
+            if ((act >> e) & 1u) dst[p + e] = v[e];
+    }
+};
 
 // Asynchronous global->shared copies (cp.async, cached in L1 so that neighbouring threads'
 // in-plane reads of the same plane still hit L1): one V-vector of T, 16 bytes (8 for 2-float
@@ -281,9 +290,13 @@ __device__ __forceinline__ void interior_vector(const StencilArgs<T>& a, const T
 // 2*kStages*16 bytes in flight without a block barrier.  For small levels the chunk is a
 // single plane (one point-vector per thread).  NORM adds the max-norm of the residual
 // over the whole shape.
-template <typename T, int OP, bool NORM, bool ONE = false>
-__device__ __forceinline__ void stencil_tile(const StencilArgs<T>& a, const int bx, const int by) {
+//
+// Args adds to StencilArgs what the results are written with (put: the whole vector, or the
+// elements in `act`); NORM_STORED: the norm covers the stored r outside the bounds too.
+template <typename T, int OP, bool NORM, bool ONE = false, typename Args = StencilArgs<T>>
+__device__ __forceinline__ void stencil_tile(const Args& a, const int bx, const int by) {
     constexpr int V = VecT<T>::V;
+    constexpr bool NORM_STORED = NORM && Args::kStored;
     __shared__ __align__(16) T stage_u[kStages][256 * V];
     // f; with NORM, the stored r in place of f at the vector's unrelaxed points
     __shared__ __align__(16) T stage_f[kStages][256 * V];
@@ -316,7 +329,7 @@ __device__ __forceinline__ void stencil_tile(const StencilArgs<T>& a, const int 
         // relaxation bounds, which counts too (infinity_norm runs over the whole shape,
         // devicearray.h:221-237): the march's own vectors' unrelaxed lanes inside it, and here
         // the planes and rows it does not march.
-        if (NORM) {
+        if (NORM_STORED) {
             if (!inr) {  // a row outside the bounds: every plane of the chunk, 4 loads in flight
                 for (int i = ia; i < ib; i += 4) {
                     T v[4][V];
@@ -413,7 +426,7 @@ __device__ __forceinline__ void stencil_tile(const StencilArgs<T>& a, const int 
                     const T left = ldg(src + p - 1), right = ldg(src + p + V);
                     interior_vector<T, OP, NORM, V>(a, vm, vc, vp, fc, ym, yp, left, right, i + j + kb + G.poff, cur,
                                                     mx);
-                    stv(a.dst + p, cur);
+                    a.put(p, i, j, kb, cur);
 #pragma unroll
                     for (int e = 0; e < V; e++) {
                         vmo[e] = vc[e];
@@ -499,7 +512,7 @@ __device__ __forceinline__ void stencil_tile(const StencilArgs<T>& a, const int 
                         }
                     }
                     T* out = a.dst + p;
-                    if (NORM && (ins & ~inr)) {  // stored r at this vector's unrelaxed points
+                    if (NORM_STORED && (ins & ~inr)) {  // stored r at this vector's unrelaxed points
                         T v[V];
                         ldv(v, out);
 #pragma unroll
@@ -510,11 +523,9 @@ __device__ __forceinline__ void stencil_tile(const StencilArgs<T>& a, const int 
                         // the whole vector is this thread's; untouched entries keep their value
                         stv(out, cur);
                     } else if (act == full) {
-                        stv(out, cur);
+                        a.put(p, i, j, kb, cur);
                     } else {
-#pragma unroll
-                        for (int e = 0; e < V; e++)
-                            if ((act >> e) & 1u) out[e] = cur[e];
+                        a.put(p, i, j, kb, cur, act);
                     }
                 }
 #pragma unroll
@@ -1420,136 +1431,76 @@ __global__ void __launch_bounds__(256) k_norm(const T* __restrict__ a, Geom G, u
 // mirror) is solved on an inner hierarchy of type Ti, then u += e.
 //
 // k_refine_residual: r = f - A u (the reference's residual with its ghost rule) over the
-// relaxation bounds; writes (Ti) r into the inner right-hand side, zeroes the inner initial
-// guess, reduces max |r|, and with WRITE_R also stores r (the user-visible residual).
-template <typename T, typename Ti>
-struct RefineArgs {
-    Geom G;                 // outer level 0
-    const T* u;
-    const T* f;
-    T* r;
-    Faces<T> F;
-    T two_h, hsq, inv_hsq;
-    int hsq_pow2;
-    int ichunk;
-    long long sxi, syi;     // inner level-0 strides
-    Ti* fi;                 // inner right-hand side
-    Ti* ui;                 // inner initial guess (zeroed) / correction (read by the update)
-    unsigned long long* norm;
-};
+// relaxation bounds, and max |r|.  Either stores r (R: the user-visible residual) or starts the
+// next correction: (Ti) r into the inner right-hand side, the inner initial guess zeroed, and,
+// with `first`, the inner level's first sweep of that zero guess (every value it reads is zero,
+// the inner boundary data included, so it is a pointwise function of the right-hand side;
+// Jacobi into the other buffer `uw`, red-black the points of one colour in place).
+//
+// The march is stencil_tile's (planes staged by cp.async, face-free body for whole warps); the
+// unstaged march this had before took 127 us on 513x257x129 with FP32 corrections (148 us with r
+// stored) and left the first sweep, 52 us, to a pass of its own.  Four refinement V-cycles there
+// 2.95 -> 2.58 ms, two F-cycles on 1025x1025x513 81.5 -> 75.9 ms.
+template <typename T, typename Ti, bool R>
+struct RefineArgs : StencilArgs<T> {
+    long long sxi, syi;  // inner level-0 strides
+    Ti* fi;              // inner right-hand side
+    Ti* ui;              // inner initial guess (zeroed)
+    Ti* uw;              // first == 1: the other Jacobi buffer
+    int first;           // 0 none, 1 Jacobi, 2 red-black
+    int fcolour;         // red-black colour of the half-sweep
+    Ti w0, w1, hsqi;     // 1 - omega, omega/6, h*h of the inner level
 
-template <typename T, typename Ti, bool WRITE_R>
-__device__ __forceinline__ void refine_residual_tile(const RefineArgs<T, Ti>& a, const int bx, const int by) {
-    constexpr int V = VecT<T>::V;
-    const Geom& G = a.G;
-    const int nv = (G.nz + V - 1) / V;
-    const int t = bx * 256 + threadIdx.x;
-    const int ia = by * a.ichunk;
-    const int ib = min(G.nx, ia + a.ichunk);
-    unsigned long long mx = 0ull;
-    if (t < G.ny * nv) {
-        const int j = t / nv;
-        const int kb = (t - j * nv) * V;
-        const long long bjk = (long long)j * G.sy + kb;
-        const long long bjki = (long long)j * a.syi + kb;
-        const bool jin = j >= G.y0 && j < G.y1;
-        unsigned ins = 0u, inr = 0u;
+    static constexpr bool kStored = false;
+    static constexpr int V = VecT<T>::V;
+    __device__ __forceinline__ Ti sweep0(Ti f) const {
+        const Ti z = Ti(0);
+        return w0 * z + w1 * (z - hsqi * f);
+    }
+    __device__ __forceinline__ void put(long long p, int i, int j, int kb, const T (&v)[V]) const {
+        if (R) {
+            stv(this->dst + p, v);
+            return;
+        }
+        const long long q = (long long)i * sxi + (long long)j * syi + kb;
+        Ti f[V], u[V];
 #pragma unroll
         for (int e = 0; e < V; e++) {
-            const int k = kb + e;
-            if (k < G.nz) ins |= 1u << e;
-            if (jin && k >= G.z0 && k < G.z1) inr |= 1u << e;
+            f[e] = (Ti)v[e];
+            const bool act = first == 2 && ((i + j + kb + e + this->G.poff) & 1) == fcolour;
+            u[e] = act ? sweep0(f[e]) : Ti(0);
         }
-        const int i0 = max(ia, G.x0);
-        const int i1 = inr ? min(ib, G.x1) : i0;
-        if (i0 < i1) {
-            const T two_h = a.two_h, m2h = -a.two_h;
-            T vm[V], vc[V], vp[V], vpp[V], fc[V], fn[V];
-            ldv(vc, a.u + (long long)i0 * G.sx + bjk);
-            if (i0 > 0) {
-                ldv(vm, a.u + (long long)(i0 - 1) * G.sx + bjk);
-            } else {
-                T v1[V];
-                ldv(v1, a.u + G.sx + bjk);
+        stv(fi + q, f);
+        stv(ui + q, u);
+        if (first == 1) {
 #pragma unroll
-                for (int e = 0; e < V; e++)
-                    vm[e] = ((ins >> e) & 1u) ? m2h * ldg(a.F.g[F_WEST] + (long long)j * G.nz + kb + e) + v1[e] : T(0);
-            }
-            if (i0 + 1 < G.nx) ldv(vp, a.u + (long long)(i0 + 1) * G.sx + bjk);
-            ldv(fc, a.f + (long long)i0 * G.sx + bjk);
-            for (int i = i0; i < i1; i++) {
-                const long long p = (long long)i * G.sx + bjk;
-                if (i + 1 < i1) {
-                    if (i + 2 < G.nx) ldv(vpp, a.u + p + 2 * G.sx);
-                    ldv(fn, a.f + p + G.sx);
-                }
-                if (i + 1 == G.nx) {
-#pragma unroll
-                    for (int e = 0; e < V; e++)
-                        vp[e] = ((ins >> e) & 1u) ? two_h * ldg(a.F.g[F_EAST] + (long long)j * G.nz + kb + e) + vm[e]
-                                                  : T(0);
-                }
-                T ym[V], yp[V];
-                if (j > 0) {
-                    ldv(ym, a.u + p - G.sy);
-                } else {
-                    T w[V];
-                    ldv(w, a.u + p + G.sy);
-#pragma unroll
-                    for (int e = 0; e < V; e++)
-                        ym[e] = ((ins >> e) & 1u) ? m2h * ldg(a.F.g[F_SOUTH] + (long long)i * G.nz + kb + e) + w[e] : T(0);
-                }
-                if (j < G.ny - 1) {
-                    ldv(yp, a.u + p + G.sy);
-                } else {
-                    T w[V];
-                    ldv(w, a.u + p - G.sy);
-#pragma unroll
-                    for (int e = 0; e < V; e++)
-                        yp[e] = ((ins >> e) & 1u) ? two_h * ldg(a.F.g[F_NORTH] + (long long)i * G.nz + kb + e) + w[e]
-                                                  : T(0);
-                }
-                const T left = kb > 0 ? ldg(a.u + p - 1) : T(0);
-                const T right = kb + V < G.nz ? ldg(a.u + p + V) : T(0);
-                T rv[V];
-#pragma unroll
-                for (int e = 0; e < V; e++) {
-                    rv[e] = T(0);
-                    if (!((inr >> e) & 1u)) continue;
-                    const int k = kb + e;
-                    const T below = e > 0 ? vc[e - 1] : left;
-                    const T above = e < V - 1 ? vc[e + 1] : right;
-                    const T zm = k > 0 ? below : m2h * ldg(a.F.g[F_BOTTOM] + (long long)i * G.ny + j) + vc[1];
-                    const T zp = k < G.nz - 1 ? above : two_h * ldg(a.F.g[F_TOP] + (long long)i * G.ny + j) + below;
-                    const T sum = vm[e] + vp[e] + ym[e] + yp[e] + zm + zp;
-                    rv[e] = residual_pt(fc[e], sum, vc[e], a.hsq, a.inv_hsq, a.hsq_pow2);
-                    mx = max(mx, abs_bits(rv[e]));
-                }
-                const long long q = (long long)i * a.sxi + bjki;
-#pragma unroll
-                for (int e = 0; e < V; e++) {
-                    if (!((inr >> e) & 1u)) continue;
-                    a.fi[q + e] = (Ti)rv[e];
-                    a.ui[q + e] = Ti(0);
-                    if (WRITE_R) a.r[p + e] = rv[e];
-                }
-#pragma unroll
-                for (int e = 0; e < V; e++) {
-                    vm[e] = vc[e];
-                    vc[e] = vp[e];
-                    vp[e] = vpp[e];
-                    fc[e] = fn[e];
-                }
-            }
+            for (int e = 0; e < V; e++) u[e] = sweep0(f[e]);
+            stv(uw + q, u);
         }
     }
-    block_max_to(mx, a.norm);
-}
+    __device__ __forceinline__ void put(long long p, int i, int j, int kb, const T (&v)[V], unsigned act) const {
+        const long long q = (long long)i * sxi + (long long)j * syi + kb;
+#pragma unroll
+        for (int e = 0; e < V; e++) {
+            if (!((act >> e) & 1u)) continue;
+            if (R) {
+                this->dst[p + e] = v[e];
+                continue;
+            }
+            const Ti f = (Ti)v[e];
+            const bool on = first == 2 && ((i + j + kb + e + this->G.poff) & 1) == fcolour;
+            fi[q + e] = f;
+            ui[q + e] = on ? sweep0(f) : Ti(0);
+            if (first == 1) uw[q + e] = sweep0(f);
+        }
+    }
+};
 
-template <typename T, typename Ti, bool WRITE_R>
-__global__ void __launch_bounds__(256) k_refine_residual(RefineArgs<T, Ti> a) {
+// Held to 64 registers, 4 blocks per SM, like the residual with its norm.
+template <typename T, typename Ti, bool R>
+__global__ void __launch_bounds__(256, 4) k_refine_residual(const __grid_constant__ RefineArgs<T, Ti, R> a) {
     pdl_begin();
-    refine_residual_tile<T, Ti, WRITE_R>(a, blockIdx.x, blockIdx.y);
+    stencil_tile<T, OP_RESIDUAL, true, false, RefineArgs<T, Ti, R>>(a, blockIdx.x, blockIdx.y);
 }
 
 // u += (T) e over the relaxation bounds (e: the inner level-0 solution).
