@@ -608,6 +608,24 @@ int short_march_chunks(const Geom& G, int bx, int cap, int chunks) {
     return chunks;
 }
 
+// Planes per block of the register form (k_stencil_planes), 0: the staged march.  `ichunk`: the
+// march's built-in planes per block.  Measured on B200 per launch, march against registers:
+// short marches on large levels, three planes -- 513x257x129 FP64 sweep 83.4 -> 77.4 us, red-black
+// half-sweep 81.3 -> 77.9, FP32 sweep 52.2 -> 46.9, residual 58.3 -> 52.7, 257^3 FP32 sweep
+// 43.5 -> 38.2 us; four planes are slower (80.3 us at 513x257x129), and the FP64 residual there
+// keeps the march (83.9 against 85.3 us).  Longer marches on levels below that, two planes --
+// 257x129x65 FP64 sweep 14.3 -> 11.0 us, half-sweep 11.9 -> 10.4, residual 14.2 -> 12.3, FP32 sweep
+// 10.0 -> 8.7; one plane per block (the ONE form) 11.6.  Where one plane fills the chip the long
+// march stays.
+template <typename T, int OP>
+int planes_in_registers(const Geom& G, int ichunk, bool built_in) {
+    if (!built_in || ichunk == 1) return 0;
+    if ((long long)G.nx * G.ny * G.nz < kShortMarchMinPoints) return 2;
+    constexpr int kShort = sizeof(T) == 8 ? 4 : 3;
+    if (ichunk > kShort || (OP == OP_RESIDUAL && sizeof(T) == 8)) return 0;
+    return 3;
+}
+
 template <typename T, int OP>
 int launch_stencil(mgp_solver* s, int l, const void* src, void* dst, T omega, int colour, unsigned long long* norm) {
     LevelState& L = s->lv[l];
@@ -630,12 +648,14 @@ int launch_stencil(mgp_solver* s, int l, const void* src, void* dst, T omega, in
     const int plane = L.G.ny * ((L.G.nz + V - 1) / V);  // threads per plane
     const int bx = (plane + kThreads - 1) / kThreads;
     int chunks = 1;
+    bool built_in = true;
     if (OP != OP_GS_COLUMN) {
         const bool nrm = OP == OP_RESIDUAL && norm;
         const int planes = L.tune[OP == OP_RESIDUAL ? (nrm ? MGP_TUNE_NORM_PLANES : MGP_TUNE_RESID_PLANES)
                                                     : MGP_TUNE_RELAX_PLANES];
         if (planes > 0) {
             chunks = (L.G.nx + planes - 1) / planes;
+            built_in = false;
         } else {
             const int cap = sm_count(s->device) *
                             (nrm ? (std::is_same<T, double>::value ? resident_blocks(k_residual_norm64<false>)
@@ -648,6 +668,21 @@ int launch_stencil(mgp_solver* s, int l, const void* src, void* dst, T omega, in
     a.ichunk = (L.G.nx + chunks - 1) / chunks;
     chunks = (L.G.nx + a.ichunk - 1) / a.ichunk;
     dim3 grid(bx, chunks);
+    if constexpr (OP != OP_GS_COLUMN) {
+        const int P = planes_in_registers<T, OP>(L.G, a.ichunk, built_in);
+        if (P) {
+            a.ichunk = P;
+            const dim3 g(bx, (L.G.nx + P - 1) / P);
+            if constexpr (OP == OP_RESIDUAL) {
+                if (norm && P == 2) return launch_k(s, k_stencil_planes<T, OP, true, 2>, g, dim3(kThreads), 0, a);
+                if constexpr (std::is_same<T, float>::value)
+                    if (norm) return launch_k(s, k_stencil_planes<T, OP, true, 3>, g, dim3(kThreads), 0, a);
+            }
+            if (P == 2) return launch_k(s, k_stencil_planes<T, OP, false, 2>, g, dim3(kThreads), 0, a);
+            if constexpr (!(OP == OP_RESIDUAL && std::is_same<T, double>::value))
+                return launch_k(s, k_stencil_planes<T, OP, false, 3>, g, dim3(kThreads), 0, a);
+        }
+    }
     if constexpr (std::is_same<T, double>::value && OP == OP_RESIDUAL) {
         if (norm) {
             if (a.ichunk == 1) return launch_k(s, k_residual_norm64<true>, grid, dim3(kThreads), 0, a);

@@ -294,7 +294,7 @@ __device__ __forceinline__ void interior_vector(const StencilArgs<T>& a, const T
 // Args adds to StencilArgs what the results are written with (put: the whole vector, or the
 // elements in `act`); NORM_STORED: the norm covers the stored r outside the bounds too.
 template <typename T, int OP, bool NORM, bool ONE = false, typename Args = StencilArgs<T>>
-__device__ __forceinline__ void stencil_tile(const Args& a, const int bx, const int by) {
+__device__ __forceinline__ unsigned long long stencil_body(const Args& a, const int bx, const int by) {
     constexpr int V = VecT<T>::V;
     constexpr bool NORM_STORED = NORM && Args::kStored;
     __shared__ __align__(16) T stage_u[kStages][256 * V];
@@ -540,7 +540,74 @@ __device__ __forceinline__ void stencil_tile(const Args& a, const int bx, const 
             cp_async_wait<0>();
         }
     }
+    return mx;
+}
+
+template <typename T, int OP, bool NORM, bool ONE = false, typename Args = StencilArgs<T>>
+__device__ __forceinline__ void stencil_tile(const Args& a, const int bx, const int by) {
+    const unsigned long long mx = stencil_body<T, OP, NORM, ONE, Args>(a, bx, by);
     if (NORM) block_max_to(mx, a.norm);
+}
+
+// P planes per block, held in registers: a thread on a face-free vector loads u of its planes and
+// the two beside them, and f, straight into registers (2P + 2 vectors in flight), and takes the
+// k-1 / k+V values from the neighbouring lanes.  What bounds the march above is the L1 data path,
+// not HBM: staging puts every vector of u and f through shared memory (a write and a read more)
+// and the two scalar loads beside a vector cost as many wavefronts as the vector, since their
+// lanes are 16 bytes apart.  Vectors on faces and blocks at the x faces take the march.
+template <typename T, int OP, bool NORM, int P, typename Args = StencilArgs<T>>
+__device__ __forceinline__ void stencil_planes(const Args& a, const int bx, const int by) {
+    constexpr int V = VecT<T>::V;
+    const Geom& G = a.G;
+    const int nv = (G.nz + V - 1) / V;
+    const int t = bx * 256 + threadIdx.x;
+    const int i0 = by * P;
+    unsigned long long mx = 0ull;
+    // interior vectors come first (plane_vector): whole warps of them
+    const int ni = nv - 2;
+    const bool fast = i0 >= 1 && i0 + P < G.nx && ni >= 1 && t < G.ny * ni;
+    int j = 0, kv = 0;
+    if (fast) {
+        j = t / ni;
+        kv = 1 + t - j * ni;
+    }
+    // (a warp's interior rows are all off the y faces or the warp takes the march)
+    if (__all_sync(0xffffffffu, fast && j >= 1 && j <= G.ny - 2)) {
+        const int kb = kv * V;
+        const long long p0 = (long long)i0 * G.sx + (long long)j * G.sy + kb;
+        const T* src = a.src + p0;
+        const T* f = a.f + p0;
+        T u[P + 2][V], fc[P][V];
+#pragma unroll
+        for (int q = 0; q < P + 2; q++) ldv(u[q], src + (q - 1) * G.sx);
+#pragma unroll
+        for (int q = 0; q < P; q++) ldv(fc[q], f + q * G.sx);
+        const int lane = threadIdx.x & 31;
+        const bool l_own = lane == 0 || kv == 1, r_own = lane == 31 || kv == nv - 2;
+#pragma unroll
+        for (int q = 0; q < P; q++) {
+            const T* s = src + q * G.sx;
+            T ym[V], yp[V], cur[V];
+            ldv(ym, s - G.sy);
+            ldv(yp, s + G.sy);
+            T left = __shfl_up_sync(0xffffffffu, u[q + 1][V - 1], 1), right = __shfl_down_sync(0xffffffffu, u[q + 1][0], 1);
+            if (l_own) left = ldg(s - 1);
+            if (r_own) right = ldg(s + V);
+            interior_vector<T, OP, NORM, V>(a, u[q], u[q + 1], u[q + 2], fc[q], ym, yp, left, right,
+                                            i0 + q + j + kb + G.poff, cur, mx);
+            a.put(p0 + q * G.sx, i0 + q, j, kb, cur);
+        }
+    } else {
+        mx = stencil_body<T, OP, NORM, false, Args>(a, bx, by);
+    }
+    if (NORM) block_max_to(mx, a.norm);
+}
+
+// 64 registers, 4 blocks per SM (five blocks at 48 spill: level-0 FP64 sweep 85 us with two planes)
+template <typename T, int OP, bool NORM, int P>
+__global__ void __launch_bounds__(256, 4) k_stencil_planes(const __grid_constant__ StencilArgs<T> a) {
+    pdl_begin();
+    stencil_planes<T, OP, NORM, P>(a, blockIdx.x, blockIdx.y);
 }
 
 template <typename T, int OP, bool NORM, bool ONE = false>
