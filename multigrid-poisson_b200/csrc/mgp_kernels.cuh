@@ -294,7 +294,7 @@ __device__ __forceinline__ void interior_vector(const StencilArgs<T>& a, const T
 // Args adds to StencilArgs what the results are written with (put: the whole vector, or the
 // elements in `act`); NORM_STORED: the norm covers the stored r outside the bounds too.
 template <typename T, int OP, bool NORM, bool ONE = false, typename Args = StencilArgs<T>>
-__device__ __forceinline__ unsigned long long stencil_body(const Args& a, const int bx, const int by) {
+__device__ __forceinline__ unsigned long long stencil_body(const Args& a, const int bx, const int ia, const int ib) {
     constexpr int V = VecT<T>::V;
     constexpr bool NORM_STORED = NORM && Args::kStored;
     __shared__ __align__(16) T stage_u[kStages][256 * V];
@@ -303,8 +303,6 @@ __device__ __forceinline__ unsigned long long stencil_body(const Args& a, const 
     const Geom& G = a.G;
     const int nv = (G.nz + V - 1) / V;
     const int t = bx * 256 + threadIdx.x;
-    const int ia = by * a.ichunk;
-    const int ib = min(G.nx, ia + a.ichunk);
     unsigned long long mx = 0ull;
     if (t < G.ny * nv) {
         int j, kv;
@@ -545,7 +543,8 @@ __device__ __forceinline__ unsigned long long stencil_body(const Args& a, const 
 
 template <typename T, int OP, bool NORM, bool ONE = false, typename Args = StencilArgs<T>>
 __device__ __forceinline__ void stencil_tile(const Args& a, const int bx, const int by) {
-    const unsigned long long mx = stencil_body<T, OP, NORM, ONE, Args>(a, bx, by);
+    const int ia = by * a.ichunk;
+    const unsigned long long mx = stencil_body<T, OP, NORM, ONE, Args>(a, bx, ia, min(a.G.nx, ia + a.ichunk));
     if (NORM) block_max_to(mx, a.norm);
 }
 
@@ -598,12 +597,79 @@ __device__ __forceinline__ void stencil_planes(const Args& a, const int bx, cons
             a.put(p0 + q * G.sx, i0 + q, j, kb, cur);
         }
     } else {
-        mx = stencil_body<T, OP, NORM, false, Args>(a, bx, by);
+        mx = stencil_body<T, OP, NORM, false, Args>(a, bx, i0, min(G.nx, i0 + P));
     }
     if (NORM) block_max_to(mx, a.norm);
 }
 
-// 64 registers, 4 blocks per SM (five blocks at 48 spill: level-0 FP64 sweep 85 us with two planes)
+// The same over a longer chunk (the batch engine's tiles): groups of P planes, the two planes
+// shared with the next group kept, its u and f loaded while the group's results are formed.
+template <typename T, int OP, bool NORM, int P, typename Args = StencilArgs<T>>
+__device__ __forceinline__ void stencil_planes_run(const Args& a, const int bx, const int by) {
+    constexpr int V = VecT<T>::V;
+    const Geom& G = a.G;
+    const int nv = (G.nz + V - 1) / V, ni = nv - 2;
+    const int t = bx * 256 + threadIdx.x;
+    const int ia = by * a.ichunk, ib = min(G.nx, ia + a.ichunk);
+    unsigned long long mx = 0ull;
+    // the chunk's planes off the x faces, in whole groups
+    const int lo = max(ia, 1), n = max(0, min(ib, G.nx - 1) - lo) / P * P;
+    const bool fast = n > 0 && ni >= 1 && t < G.ny * ni;
+    int j = 0, kv = 0;
+    if (fast) {
+        j = t / ni;
+        kv = 1 + t - j * ni;
+    }
+    const bool lanes = __all_sync(0xffffffffu, fast && j >= 1 && j <= G.ny - 2);
+    if (lanes) {
+        const int kb = kv * V;
+        long long p0 = (long long)lo * G.sx + (long long)j * G.sy + kb;
+        T u[P + 2][V], fc[P][V];
+        ldv(u[P], a.src + p0 - G.sx);
+        ldv(u[P + 1], a.src + p0);
+        const int lane = threadIdx.x & 31;
+        const bool l_own = lane == 0 || kv == 1, r_own = lane == 31 || kv == nv - 2;
+#pragma unroll 1
+        for (int i = lo; i < lo + n; i += P, p0 += P * G.sx) {
+            const T* src = a.src + p0;
+#pragma unroll
+            for (int e = 0; e < V; e++) {
+                u[0][e] = u[P][e];
+                u[1][e] = u[P + 1][e];
+            }
+#pragma unroll
+            for (int q = 0; q < P; q++) ldv(u[q + 2], src + (q + 1) * G.sx);
+#pragma unroll
+            for (int q = 0; q < P; q++) ldv(fc[q], a.f + p0 + q * G.sx);
+#pragma unroll
+            for (int q = 0; q < P; q++) {
+                const T* s = src + q * G.sx;
+                T ym[V], yp[V], cur[V];
+                ldv(ym, s - G.sy);
+                ldv(yp, s + G.sy);
+                T left = __shfl_up_sync(0xffffffffu, u[q + 1][V - 1], 1);
+                T right = __shfl_down_sync(0xffffffffu, u[q + 1][0], 1);
+                if (l_own) left = ldg(s - 1);
+                if (r_own) right = ldg(s + V);
+                interior_vector<T, OP, NORM, V>(a, u[q], u[q + 1], u[q + 2], fc[q], ym, yp, left, right,
+                                                i + q + j + kb + G.poff, cur, mx);
+                a.put(p0 + q * G.sx, i + q, j, kb, cur);
+            }
+        }
+    }
+    // what is left: the planes before and after the groups, or all of them
+    int a0 = ia, a1 = lanes ? lo : ib;
+#pragma unroll 1
+    for (int part = 0; part < 2; part++) {
+        if (a0 < a1) mx = max(mx, stencil_body<T, OP, NORM, false, Args>(a, bx, a0, a1));
+        a0 = lanes ? lo + n : ib;
+        a1 = ib;
+    }
+    if (NORM) block_max_to(mx, a.norm);
+}
+
+// 64 registers, 4 blocks per SM (five blocks at 48 spill: 513x257x129 FP64 sweep 85 us with two
+// planes per block)
 template <typename T, int OP, bool NORM, int P>
 __global__ void __launch_bounds__(256, 4) k_stencil_planes(const __grid_constant__ StencilArgs<T> a) {
     pdl_begin();
