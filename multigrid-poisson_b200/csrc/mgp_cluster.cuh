@@ -44,8 +44,8 @@ struct ClLevel {
     T two_h, hsq, inv_hsq, one_omega, omega_sixth, h;
     int pow2;
     int P, nact;       // planes per CTA; CTAs that own planes
-    int pl;            // points per plane
-    unsigned m_nz, m_ny, m_pl, m_P;  // cl_div's magic numbers
+    int rp, pl;            // row pitch in shared memory (even) and elements of a plane
+    unsigned m_nz, m_ny, m_yz, m_rp, m_pl, m_P;  // cl_div's magic numbers
     int ncol;          // relaxed columns (points of a plane inside the y and z bounds)
     int nitem;         // work items of a relaxation: columns, or pairs of columns (red-black)
     int nseg, seglen;  // an item's planes are split over nseg threads, seglen planes each
@@ -82,6 +82,11 @@ __device__ __forceinline__ void cl_sync() {
     if (threadIdx.x == 0) asm volatile("fence.acq_rel.cluster;" ::: "memory");
     __syncwarp();
     asm volatile("barrier.cluster.arrive.relaxed.aligned;\nbarrier.cluster.wait.acquire.aligned;\n" ::: "memory");
+}
+// The same before data of a level go to another one, unless both levels sit in one CTA.
+__device__ __forceinline__ void cl_sync_levels(int nact_a, int nact_b) {
+    if (nact_a == 1 && nact_b == 1) __syncthreads();
+    else cl_sync();
 }
 __device__ __forceinline__ unsigned cl_map(unsigned addr, unsigned rank) {
     unsigned a;
@@ -145,7 +150,7 @@ struct __align__(16) ClCta {
     int nitem, nseg, seglen, tab; // relaxation items; tab: byte offset of their table
     int ncol, rseg, rlen, rtab;   // the residual's columns
     int lo, hi, np, i0;           // planes [i0, i0 + np), of which [lo, hi) (counted from i0) are relaxed
-    int pl, nz, ny, nx;
+    int pl, rp, nz, ny, nx;
     unsigned la, ra;              // cluster addresses (offset 0) of the halo planes it fills, 0: no neighbour
     unsigned lmb, rmb;            // the neighbours' mbarriers for them
     unsigned bl[3], br[3];        // bytes expected from each side: colour 0, colour 1, every relaxed point
@@ -167,12 +172,13 @@ struct ClSlab {
 
 // Column table entries: the column's index in the plane and the faces it lies on.  Columns off
 // the faces come first, so whole warps take the ghost-free stencil.  Red-black relaxations work on
-// pairs of columns (k, k+1), of which one point per plane has the colour, so every lane has work:
+// pairs of columns (j, j+1), of which one point per plane has the colour, so every lane has work:
 // the entry is the first column's, with the parity of j + k + poff, whether the second column is
-// on the top face and whether there is one.
+// on the north face and whether there is one.  A warp's lanes run along k and alternate between
+// the two rows; with an even row pitch their addresses fall into different banks.
 enum : unsigned {
     CL_SOUTH = 1u << 16, CL_NORTH = 1u << 17, CL_BOTTOM = 1u << 18, CL_TOP = 1u << 19,
-    CL_ODD = 1u << 20, CL_TOP2 = 1u << 21, CL_ONE = 1u << 22
+    CL_ODD = 1u << 20, CL_NORTH2 = 1u << 21, CL_ONE = 1u << 22
 };
 constexpr unsigned kClEdge = CL_SOUTH | CL_NORTH | CL_BOTTOM | CL_TOP;
 
@@ -209,6 +215,7 @@ __device__ __forceinline__ void cl_tables(const ClArgs<T>& a, unsigned char* sme
         c.lo = max(0, L.G.x0 - c.i0);
         c.hi = min(c.np, L.G.x1 - c.i0);
         c.pl = L.pl;
+        c.rp = L.rp;
         c.nz = L.G.nz;
         c.ny = L.G.ny;
         c.nx = L.G.nx;
@@ -261,17 +268,17 @@ __device__ __forceinline__ void cl_tables(const ClArgs<T>& a, unsigned char* sme
                 j = ya + q / sides;
                 k = q % sides == 0 && bottom ? 0 : G.nz - 1;
             }
-            tab[c] = (unsigned)(j * G.nz + k) | (j == 0 ? CL_SOUTH : 0u) | (j == G.ny - 1 ? CL_NORTH : 0u) |
+            tab[c] = (unsigned)(j * L.rp + k) | (j == 0 ? CL_SOUTH : 0u) | (j == G.ny - 1 ? CL_NORTH : 0u) |
                      (k == 0 ? CL_BOTTOM : 0u) | (k == G.nz - 1 ? CL_TOP : 0u);
         }
         if (JAC) continue;
         unsigned* pair = reinterpret_cast<unsigned*>(smem + L.so_pair);
-        const int np2 = (G.z1 - G.z0 + 1) / 2;  // pairs of a row
         for (int c = threadIdx.x; c < L.nitem; c += blockDim.x) {
-            const int j = G.y0 + c / np2, k = G.z0 + c % np2 * 2;
-            pair[c] = (unsigned)(j * G.nz + k) | (j == 0 ? CL_SOUTH : 0u) | (j == G.ny - 1 ? CL_NORTH : 0u) |
-                      (k == 0 ? CL_BOTTOM : 0u) | (k == G.nz - 1 ? CL_TOP : 0u) | (k + 1 == G.nz - 1 ? CL_TOP2 : 0u) |
-                      (k + 1 >= G.z1 ? CL_ONE : 0u) | (((j + k + G.poff) & 1) ? CL_ODD : 0u);
+            const int j = G.y0 + c / w * 2, k = G.z0 + c % w;
+            pair[c] = (unsigned)(j * L.rp + k) | (j == 0 ? CL_SOUTH : 0u) | (j == G.ny - 1 ? CL_NORTH : 0u) |
+                      (k == 0 ? CL_BOTTOM : 0u) | (k == G.nz - 1 ? CL_TOP : 0u) |
+                      (j + 1 == G.ny - 1 ? CL_NORTH2 : 0u) | (j + 1 >= G.y1 ? CL_ONE : 0u) |
+                      (((j + k + G.poff) & 1) ? CL_ODD : 0u);
         }
     }
 }
@@ -318,10 +325,10 @@ template <typename T>
 __device__ __forceinline__ void cl_edge(const ClArgs<T>& a, int l, const ClCta<T>& s, const T* sm, const T* u, int ii,
                                         int rem, unsigned e, T& ym, T& yp, T& zm, T& zp) {
     const int* g = a.L[l].so_g;
-    const int j = cl_div(rem, a.L[l].m_nz), k = rem - j * s.nz;
+    const int j = cl_div(rem, a.L[l].m_rp), k = rem - j * s.rp;
     const T h2 = s.two_h, m2h = -s.two_h;
-    ym = !(e & CL_SOUTH) ? u[-s.nz] : m2h * sm[g[F_SOUTH] + (ii + 1) * s.nz + k] + u[s.nz];
-    yp = !(e & CL_NORTH) ? u[s.nz] : h2 * sm[g[F_NORTH] + (ii + 1) * s.nz + k] + u[-s.nz];
+    ym = !(e & CL_SOUTH) ? u[-s.rp] : m2h * sm[g[F_SOUTH] + (ii + 1) * s.nz + k] + u[s.rp];
+    yp = !(e & CL_NORTH) ? u[s.rp] : h2 * sm[g[F_NORTH] + (ii + 1) * s.nz + k] + u[-s.rp];
     zm = !(e & CL_BOTTOM) ? u[-1] : m2h * sm[g[F_BOTTOM] + (ii + 1) * s.ny + j] + u[1];
     zp = !(e & CL_TOP) ? u[1] : h2 * sm[g[F_TOP] + (ii + 1) * s.ny + j] + u[-1];
 }
@@ -349,8 +356,8 @@ __device__ __forceinline__ void cl_march(const ClArgs<T>& a, int l, const ClCta<
         const T vp = s.i0 + ii < s.nx - 1 ? u[s.pl] : s.two_h * sm[a.L[l].so_g[F_EAST] + rem] + u[-s.pl];
         T ym, yp, zm, zp;
         if (!edge) {
-            ym = u[-s.nz];
-            yp = u[s.nz];
+            ym = u[-s.rp];
+            yp = u[s.rp];
             zm = u[-1];
             zp = u[1];
         } else {
@@ -374,16 +381,16 @@ __device__ __forceinline__ void cl_march_pair(const ClArgs<T>& a, int l, const C
     const int base = src + rem0 + lo * s.pl;
     for (int ii = lo, p = base; ii < hi; ii++, p += s.pl, second ^= 1) {
         if (second && (e & CL_ONE)) continue;
-        const int rem = rem0 + second;
-        T* u = sm + p + second;
+        const int rem = second ? rem0 + s.rp : rem0;
+        T* u = sm + (second ? p + s.rp : p);
         const T fv = sm[s.f + rem + ii * s.pl];
         const T vm = s.i0 + ii > 0 ? u[-s.pl] : -s.two_h * sm[a.L[l].so_g[F_WEST] + rem] + u[s.pl];
         const T vp = s.i0 + ii < s.nx - 1 ? u[s.pl] : s.two_h * sm[a.L[l].so_g[F_EAST] + rem] + u[-s.pl];
         T ym, yp, zm, zp;
-        const unsigned ee = second ? (e & (CL_SOUTH | CL_NORTH)) | ((e & CL_TOP2) ? CL_TOP : 0u) : e & kClEdge;
+        const unsigned ee = second ? (e & (CL_BOTTOM | CL_TOP)) | ((e & CL_NORTH2) ? CL_NORTH : 0u) : e & kClEdge;
         if (!ee) {
-            ym = u[-s.nz];
-            yp = u[s.nz];
+            ym = u[-s.rp];
+            yp = u[s.rp];
             zm = u[-1];
             zp = u[1];
         } else {
@@ -509,23 +516,23 @@ __device__ __forceinline__ void cl_face_restrict(const ClArgs<T>& a, int l, T* s
     if (fc == F_EAST || fc == F_WEST) {
         const int x = upper ? G.nx - 1 : 0;
         if (x < S.i0 || x >= S.i0 + S.np) return;
-        for (int t = t0; t < C.pl; t += nthr) {
+        for (int t = t0; t < Gc.ny * Gc.nz; t += nthr) {
             const int J = cl_div(t, C.m_nz), K = t - J * Gc.nz;
             T g;
             if (a.fw) {
                 const int jj = min(G.ny - 1, 2 * J), kk = min(G.nz - 1, 2 * K);
-                auto A = [&](int, int y, int z) -> double { return (double)gf[y * G.nz + z]; };
+                auto A = [&](int, int y, int z) -> double { return (double)gf[y * F.rp + z]; };
                 g = fw_sum<T>(A, 0, 0, 0, max(0, jj - 1), jj, min(G.ny - 1, jj + 1), max(0, kk - 1), kk,
                               min(G.nz - 1, kk + 1));
             } else {
-                g = gf[2 * J * G.nz + 2 * K];
+                g = gf[2 * J * F.rp + 2 * K];
             }
-            const int idx = 2 * J * G.nz + 2 * K;
+            const int idx = 2 * J * F.rp + 2 * K;
             // planes x, x+d and x+2d: in the slab or its halo, as slabs hold at least two planes
             const T* up = sm + so_u + (x - S.i0 + 1) * F.pl + idx;
             g -= (c1 * up[0] + c2 * up[d * F.pl] + c3 * up[2 * d * F.pl]) / F.h;
             const int owner = upper ? C.nact - 1 : 0;
-            cl_st(cl_map(sbase + (unsigned)(C.so_g[fc] + t) * (unsigned)sizeof(T), owner), g);
+            cl_st(cl_map(sbase + (unsigned)(C.so_g[fc] + J * C.rp + K) * (unsigned)sizeof(T), owner), g);
         }
     } else {
         const bool ns = fc == F_NORTH || fc == F_SOUTH;  // rows along k, else rows along j
@@ -546,9 +553,9 @@ __device__ __forceinline__ void cl_face_restrict(const ClArgs<T>& a, int l, T* s
             } else {
                 g = gf[sl * len + 2 * q];
             }
-            const int at = ns ? (upper ? (G.ny - 1) * G.nz : 0) + 2 * q : 2 * q * G.nz + (upper ? G.nz - 1 : 0);
+            const int at = ns ? (upper ? (G.ny - 1) * F.rp : 0) + 2 * q : 2 * q * F.rp + (upper ? G.nz - 1 : 0);
             const T* up = sm + so_u + sl * F.pl + at;
-            const int s = d * (ns ? G.nz : 1);
+            const int s = d * (ns ? F.rp : 1);
             g -= (c1 * up[0] + c2 * up[s] + c3 * up[2 * s]) / F.h;
             cl_put(C, sbase, C.so_g[fc], clen, I, q, g);
         }
@@ -580,26 +587,27 @@ __device__ __forceinline__ void cl_setup(const ClArgs<T>& a, int l, T* sm, unsig
     if (np > 0) {
         const int I0 = (i0 + 1) >> 1, I1 = (i0 + np + 1) >> 1;
         const T* r = sm + F.so_r;
-        const int n = (I1 - I0) * C.pl;
+        const int yz = C.G.ny * C.G.nz, n = (I1 - I0) * yz;
         for (int t = threadIdx.x; t < n; t += blockDim.x) {
-            const int q = cl_div(t, C.m_pl), rem = t - q * C.pl;
-            const int I = I0 + q, J = cl_div(rem, C.m_nz), K = rem - J * C.G.nz;
+            const int q = cl_div(t, C.m_yz), d = t - q * yz;
+            const int I = I0 + q, J = cl_div(d, C.m_nz), K = d - J * C.G.nz;
+            const int rem = J * C.rp + K;
             const int sl = 2 * I - i0 + 1;
             T v;
             if (a.fw) {
                 const int im = (2 * I > 0 ? sl - 1 : sl) * F.pl, ic = sl * F.pl, ip = (2 * I < G.nx - 1 ? sl + 1 : sl) * F.pl;
                 const int jj = min(G.ny - 1, 2 * J), kk = min(G.nz - 1, 2 * K);
-                const int jm = max(0, jj - 1) * G.nz, jp = min(G.ny - 1, jj + 1) * G.nz;
+                const int jm = max(0, jj - 1) * F.rp, jp = min(G.ny - 1, jj + 1) * F.rp;
                 auto A = [&](int x, int y, int z) -> double { return (double)r[x + y + z]; };
-                v = fw_sum<T>(A, im, ic, ip, jm, jj * G.nz, jp, max(0, kk - 1), kk, min(G.nz - 1, kk + 1));
+                v = fw_sum<T>(A, im, ic, ip, jm, jj * F.rp, jp, max(0, kk - 1), kk, min(G.nz - 1, kk + 1));
             } else {
-                v = r[sl * F.pl + 2 * J * G.nz + 2 * K];
+                v = r[sl * F.pl + 2 * J * F.rp + 2 * K];
             }
             const int owner = cl_div(I, C.m_P);
             cl_st(cl_map(sbase + (unsigned)(C.so_f + (I - owner * C.P) * C.pl + rem) * (unsigned)sizeof(T), owner), v);
         }
     }
-    cl_sync();
+    cl_sync_levels(F.nact, C.nact);
     if (JAC) {
         zero_coarse();
         __syncthreads();
@@ -617,7 +625,7 @@ __device__ __forceinline__ void cl_prolong(const ClArgs<T>& a, int l, T* sm, uns
     const int ia = max(0, i0 - 1), ib = min(nx, i0 + np + 1);           // planes written
     const int Ia = ia >> 1, Ib = min(C.G.nx - 1, ((ib - 1) >> 1) + 1);  // coarse planes read
     const int plc = C.pl, so_c = C.so_u[(cur >> (l + 1)) & 1u];
-    cl_sync();  // every CTA's last sweep of the coarse level
+    cl_sync_levels(F.nact, C.nact);  // every CTA's last sweep of the coarse level
     if (np > 0) {
         const int n = (Ib - Ia + 1) * plc, Pc = C.P;
         const unsigned m_pl = C.m_pl, m_P = C.m_P;
@@ -634,7 +642,7 @@ __device__ __forceinline__ void cl_prolong(const ClArgs<T>& a, int l, T* sm, uns
         T* u = sm + F.so_u[(cur >> l) & 1u];
         T* r = sm + F.so_r;
         // an item is a pair of columns (k even, k+1): both interpolate between the same coarse rows
-        const int pl = F.pl, nz = F.G.nz, ny = F.G.ny, nzc = C.G.nz;
+        const int pl = F.pl, rpf = F.rp, rpc = C.rp, ny = F.G.ny, nzc = C.G.nz;
         const int x0 = F.G.x0, x1 = F.G.x1, y0b = F.G.y0, y1b = F.G.y1, z0 = F.G.z0, z1 = F.G.z1;
         const int items = ny * nzc;  // nz = 2*nzc - 1: the last column of a row is alone
         const unsigned m_nzc = C.m_nz;
@@ -648,8 +656,8 @@ __device__ __forceinline__ void cl_prolong(const ClArgs<T>& a, int l, T* sm, uns
             const int jp = j & 1;
             const bool pair = kc + 1 < nzc;
             const bool jin = j >= y0b && j < y1b, in0 = jin && k >= z0 && k < z1, in1 = jin && k + 1 < z1;
-            const T* c = sc + (j >> 1) * nzc + kc;
-            const int dj = jp ? nzc : 0, dk = pair ? 1 : 0;  // what is not interpolated repeats a value (unused)
+            const T* c = sc + (j >> 1) * rpc + kc;
+            const int dj = jp ? rpc : 0, dk = pair ? 1 : 0;  // what is not interpolated repeats a value (unused)
             T c0[2][2], c1[2][2];
             auto load = [&](T (&d)[2][2], int I) {
                 const T* q = c + (I - Ia) * plc;
@@ -659,8 +667,8 @@ __device__ __forceinline__ void cl_prolong(const ClArgs<T>& a, int l, T* sm, uns
                 d[1][1] = q[dj + dk];
             };
             load(c0, sa >> 1);
-            T* up = u + (sa - i0 + 1) * pl + j * nz + k;
-            T* rp = r + (sa - i0 + 1) * pl + j * nz + k;
+            T* up = u + (sa - i0 + 1) * pl + j * rpf + k;
+            T* rp = r + (sa - i0 + 1) * pl + j * rpf + k;
             for (int i = sa; i < sb; i++, up += pl, rp += pl) {
                 T x[2][2];
                 if (i & 1) {
@@ -704,7 +712,8 @@ __device__ __forceinline__ void cl_load(const ClArgs<T>& a, T* sm, int rank) {
         const int nx = L.G.nx, ny = L.G.ny, nz = L.G.nz, pl = L.pl, i0 = rank * L.P, np = min(L.P, nx - i0);
         const int x0 = L.G.x0, x1 = L.G.x1, y0 = L.G.y0, y1 = L.G.y1, z0 = L.G.z0, z1 = L.G.z1;
         const long long sx = L.G.sx, sy = L.G.sy;
-        const unsigned m_nz = L.m_nz, m_pl = L.m_pl;
+        const int rp = L.rp;
+        const unsigned m_nz = L.m_nz, m_yz = L.m_yz;
         if (np <= 0) continue;
         const int ia = max(0, i0 - 1), ib = min(nx, i0 + np + 1);
         const int c = (a.cur >> l) & 1;
@@ -716,11 +725,11 @@ __device__ __forceinline__ void cl_load(const ClArgs<T>& a, T* sm, int rank) {
         T* sp = sm + L.so_u[c ^ 1];
         T* sf = sm + L.so_f;
         T* sr = sm + L.so_r;
-        const int n = (ib - ia) * pl;
+        const int yz = ny * nz, n = (ib - ia) * yz;
         for (int t = threadIdx.x; t < n; t += blockDim.x) {
-            const int q = cl_div(t, m_pl), rem = t - q * pl;
+            const int q = cl_div(t, m_yz), rem = t - q * yz;
             const int i = ia + q, j = cl_div(rem, m_nz), k = rem - j * nz;
-            const int p = (i - i0 + 1) * pl + rem;
+            const int p = (i - i0 + 1) * pl + j * rp + k;
             const long long o = (long long)i * sx + j * sy + k;
             const bool unrelaxed = i < x0 || i >= x1 || j < y0 || j >= y1 || k < z0 || k >= z1;
             if (l == 0) {
@@ -736,7 +745,10 @@ __device__ __forceinline__ void cl_load(const ClArgs<T>& a, T* sm, int rank) {
             T* sg = sm + L.so_g[fc];
             const T* gg = L.g[fc];
             if (fc == F_EAST || fc == F_WEST) {
-                for (int t = threadIdx.x; t < pl; t += blockDim.x) cl_copy(sg + t, gg + t);
+                for (int t = threadIdx.x; t < ny * nz; t += blockDim.x) {
+                    const int j = cl_div(t, L.m_nz);
+                    cl_copy(sg + t + j * (rp - nz), gg + t);
+                }
             } else {
                 const int len = (fc == F_NORTH || fc == F_SOUTH) ? nz : ny;
                 const int m = (ib - ia) * len;
@@ -755,7 +767,8 @@ __device__ __forceinline__ void cl_store(const ClArgs<T>& a, const T* sm, int ra
         const int nx = L.G.nx, ny = L.G.ny, nz = L.G.nz, pl = L.pl, i0 = rank * L.P, np = min(L.P, nx - i0);
         const int x0 = L.G.x0, x1 = L.G.x1, y0 = L.G.y0, y1 = L.G.y1, z0 = L.G.z0, z1 = L.G.z1;
         const long long sx = L.G.sx, sy = L.G.sy;
-        const unsigned m_nz = L.m_nz, m_pl = L.m_pl;
+        const int rp = L.rp;
+        const unsigned m_nz = L.m_nz, m_yz = L.m_yz;
         if (np <= 0) continue;
         T* g0 = L.ub[0];
         T* g1 = L.ub[1];
@@ -765,16 +778,16 @@ __device__ __forceinline__ void cl_store(const ClArgs<T>& a, const T* sm, int ra
         const T* s1 = sm + L.so_u[1];
         const T* sf = sm + L.so_f;
         const T* sr = sm + L.so_r;
-        const int n = np * pl;
+        const int yz = ny * nz, n = np * yz;
         for (int t = threadIdx.x; t < n; t += blockDim.x) {
-            const int q = cl_div(t, m_pl), rem = t - q * pl;
+            const int q = cl_div(t, m_yz), rem = t - q * yz;
             const int i = i0 + q, j = cl_div(rem, m_nz), k = rem - j * nz;
-            const int p = t + pl;
+            const int p = (q + 1) * pl + j * rp + k;
             const long long o = (long long)i * sx + j * sy + k;
             g0[o] = s0[p];
             if (g1) g1[o] = s1[p];
             if (i < x0 || i >= x1 || j < y0 || j >= y1 || k < z0 || k >= z1) gr[o] = sr[p];
-            if (l > 0) gf[o] = sf[t];
+            if (l > 0) gf[o] = sf[p - pl];
         }
         if (l == 0) continue;
         for (int fc = 0; fc < 6; fc++) {
@@ -783,7 +796,7 @@ __device__ __forceinline__ void cl_store(const ClArgs<T>& a, const T* sm, int ra
             T* gg = L.g[fc];
             if (fc == F_EAST || fc == F_WEST) {
                 if (rank != (fc == F_EAST ? L.nact - 1 : 0)) continue;
-                for (int t = threadIdx.x; t < pl; t += blockDim.x) gg[t] = sg[t];
+                for (int t = threadIdx.x; t < ny * nz; t += blockDim.x) gg[t] = sg[t + cl_div(t, L.m_nz) * (rp - nz)];
             } else {
                 const int len = (fc == F_NORTH || fc == F_SOUTH) ? nz : ny;
                 for (int t = threadIdx.x; t < np * len; t += blockDim.x) gg[i0 * len + t] = sg[len + t];
@@ -831,7 +844,7 @@ __global__ void __launch_bounds__(kClMaxThreads, 1) k_cluster(const __grid_const
             cl_prolong(a, l, sm, sbase, cur, rank);
             // Jacobi's next sweep only reads this CTA's u and writes the other buffer; an in-place
             // sweep of a neighbour would write halo points still being updated here
-            if (JAC) __syncthreads();
+            if (JAC || a.L[l].nact == 1) __syncthreads();
             else cl_sync();
         } else {  // the solve loop's residual of level 0, stored, and its max-norm over the shape
             cl_residual(a, l, S[l], sm, S[l].u[(cur >> l) & 1u], X);
@@ -841,7 +854,8 @@ __global__ void __launch_bounds__(kClMaxThreads, 1) k_cluster(const __grid_const
             const Geom& G = L.G;
             unsigned long long mx = 0ull;
             for (int rem = threadIdx.x; rem < L.pl; rem += blockDim.x) {
-                const int j = cl_div(rem, L.m_nz), k = rem - j * G.nz;
+                const int j = cl_div(rem, L.m_rp), k = rem - j * L.rp;
+                if (k >= G.nz) continue;
                 for (int ii = 0; ii < np; ii++) {
                     const T v = sm[L.so_r + (ii + 1) * L.pl + rem];
                     mx = max(mx, abs_bits(v));

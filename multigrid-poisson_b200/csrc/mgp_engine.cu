@@ -1262,7 +1262,14 @@ unsigned div_magic(int d) { return d <= 1 ? 0u : (unsigned)(((1ull << 32) + d - 
 
 // Planes of a CTA's slab: at least two in every slab, the last one included (the east and west
 // face restriction reads three planes from the face inwards, two slabs' worth at most).
-int slab_planes(int nx, int nc) {
+// Levels on which a sweep updates at most kClOnePoints points go to one CTA: their sweeps then end
+// with a block barrier instead of an exchange (820 cycles, more than their arithmetic).  Ten 65^3
+// red-black F-cycles 2.55 -> 2.43 ms (9^3 and 5^3 in one CTA), four 33x17x17 Jacobi ones 375 -> 363 us
+// (9x5x5); Jacobi levels of 765 and 1001 points are faster in slabs (161x97x193 by 2%).
+constexpr long long kClOnePoints = 512;
+int slab_planes(const Geom& G, int nc, bool jacobi) {
+    const int nx = G.nx;
+    if ((long long)nx * G.ny * G.nz <= (jacobi ? kClOnePoints : 2 * kClOnePoints)) return nx;
     int P = std::max(2, (nx + nc - 1) / nc);
     while (P < nx && nx % P == 1) P++;
     return std::min(P, nx);
@@ -1278,11 +1285,12 @@ bool cluster_plan(const mgp_solver* s, int t, int nc, ClArgs<T>* a, size_t* smem
     for (int m = t; m < s->levels; m++) {
         const LevelState& L = s->lv[m];
         const Geom& G = L.G;
-        const int P = slab_planes(G.nx, nc);
-        const long long pl = (long long)G.ny * G.nz;
+        const int P = slab_planes(G, nc, jac);
+        const int rp = G.nz + (G.nz & 1);
+        const long long pl = (long long)G.ny * rp;
         if (pl * (4 * P + 6) * (long long)sizeof(T) > (long long)kClMaxSmem * 2) return false;
         const int ncol = std::max(0, G.y1 - G.y0) * std::max(0, G.z1 - G.z0);
-        const int nitem = jac ? ncol : std::max(0, G.y1 - G.y0) * ((std::max(0, G.z1 - G.z0) + 1) / 2);
+        const int nitem = jac ? ncol : (std::max(0, G.y1 - G.y0) + 1) / 2 * std::max(0, G.z1 - G.z0);
         // Threads: one per relaxation item of the finest level, or even passes over the items; an
         // operation's set-up per warp counts, so no more than that (at least 8 warps: the Neumann
         // faces are dealt out to warps).
@@ -1296,11 +1304,14 @@ bool cluster_plan(const mgp_solver* s, int t, int nc, ClArgs<T>* a, size_t* smem
         q.G = G;
         q.P = P;
         q.nact = (G.nx + P - 1) / P;
+        q.rp = rp;
         q.pl = (int)pl;
+        q.m_rp = div_magic(rp);
         q.nseg = nseg;
         q.seglen = (P + nseg - 1) / nseg;
         q.m_nz = div_magic(G.nz);
         q.m_ny = div_magic(G.ny);
+        q.m_yz = div_magic(G.ny * G.nz);
         q.m_pl = div_magic((int)pl);
         q.m_P = div_magic(P);
         q.ncol = ncol;
@@ -1325,7 +1336,7 @@ bool cluster_plan(const mgp_solver* s, int t, int nc, ClArgs<T>* a, size_t* smem
         }
         if (m > t) {
             const LevelState& F = s->lv[m - 1];
-            const int Pf = slab_planes(F.G.nx, nc);
+            const int Pf = slab_planes(F.G, nc, jac);
             gather = std::max(gather, ((Pf + 2) / 2 + 3) * pl);
         }
         if (off * (long long)sizeof(T) > (long long)kClMaxSmem) return false;
@@ -1341,7 +1352,7 @@ bool cluster_plan(const mgp_solver* s, int t, int nc, ClArgs<T>* a, size_t* smem
             a->L[m - t].so_tab = (int)bytes;
             a->L[m - t].so_pair = (int)bytes + 4 * wy * wz;
         }
-        bytes += 4ll * wy * (wz + (jac ? 0 : (wz + 1) / 2));
+        bytes += 4ll * wz * (wy + (jac ? 0 : (wy + 1) / 2));
     }
     *smem = (size_t)bytes;
     *threads = nt;
