@@ -736,11 +736,15 @@ __device__ __forceinline__ T fw_point(const T* in, const View& vi, int i, int j,
 
 // fw_point for a thread of a warp whose lanes hold consecutive coarse points t of one coarse
 // plane (t = j*n[2] + k).  Each fine row of the 3x3 neighbourhood is read as the aligned pair
-// (2k, 2k+1) in one 2-element load; the value at 2k-1 is the second element of lane-1's pair
-// when that lane holds (j, k-1), else (first lane of the warp, or k = 0) a scalar load or the
-// clamped centre.  Same values and the same sums as fw_point.  Every lane of the warp must
-// call it (lanes without a point with any point of the plane); the fine rows hold an odd
-// number of points at an even pitch, so 2k+1 lies inside the row's pitch.
+// (2k, 2k+1) in one 2-element load.  The sum of column 2k-1 has the weights and the order of the
+// sum of column 2k+1, so it is, bit for bit, the latter sum of lane-1 when that lane holds
+// (j, k-1): one shuffle instead of nine values and their sum (and, in FP32, their conversions,
+// which bound the pass).  Otherwise (first lane of the warp, or k = 0, where it is the clamped
+// centre column) the thread sums it itself.  Every lane of the warp must call it (lanes without
+// a point with any point of the plane); the fine rows hold an odd number of points at an even
+// pitch, so 2k+1 lies inside the row's pitch.
+// 513x257x129 to 257x129x65: FP64 42.2 -> 33.7 us, FP32 33.9 -> 27.2 us (with the values of
+// column 2k-1 loaded ahead, in nine more registers, 37.0 and 28.5 us).
 template <typename T>
 __device__ __forceinline__ T fw_point_pairs(const T* in, const View& vi, int i, int j, int k) {
     const int ii = min(vi.n[0] - 1, 2 * i), jj = min(vi.n[1] - 1, 2 * j), kk = 2 * k;
@@ -748,25 +752,46 @@ __device__ __forceinline__ T fw_point_pairs(const T* in, const View& vi, int i, 
     const int jm = max(0, jj - 1), jp = min(vi.n[1] - 1, jj + 1);
     const bool from_lane = (threadIdx.x & 31) != 0 && k > 0;
     const bool clamp_p = kk + 1 > vi.n[2] - 1;  // kp = kk
-    const int X[3] = {im, ii, ip}, Y[3] = {jm, jj, jp};
-    double vm[3][3], v0[3][3], vp[3][3];
+    const long long X[3] = {im * vi.s0, ii * vi.s0, ip * vi.s0}, Y[3] = {jm * vi.s1, jj * vi.s1, jp * vi.s1};
+    const T* col = in + kk;
+    T pr[3][3][2];
+#pragma unroll
+    for (int x = 0; x < 3; x++)
+#pragma unroll
+        for (int y = 0; y < 3; y++) ldv(pr[x][y], col + X[x] + Y[y]);
+    // weights (1,2,1 | 2,4,2 | 1,2,1), doubled on the centre column; fullweighting.h:82-109
+    double s_0 = 0.0, s_p = 0.0;
 #pragma unroll
     for (int x = 0; x < 3; x++)
 #pragma unroll
         for (int y = 0; y < 3; y++) {
-            const T* row = in + X[x] * vi.s0 + Y[y] * vi.s1;
-            T pr[2];
-            ldv(pr, row + kk);
-            const T prev = __shfl_up_sync(0xffffffffu, pr[1], 1);
-            v0[x][y] = (double)pr[0];
-            vp[x][y] = (double)(clamp_p ? pr[0] : pr[1]);
-            T m = pr[0];  // k = 0: km = kk
-            if (k > 0) m = from_lane ? prev : ldg(row + kk - 1);
-            vm[x][y] = (double)m;
+            const double w = (x == 1 ? 2.0 : 1.0) * (y == 1 ? 2.0 : 1.0);
+            const double a0 = (double)pr[x][y][0], ap = (double)(clamp_p ? pr[x][y][0] : pr[x][y][1]);
+            if (x == 0 && y == 0) {
+                s_0 = 2.0 * w * a0;
+                s_p = w * ap;
+            } else {
+                s_0 = s_0 + 2.0 * w * a0;
+                s_p = s_p + w * ap;
+            }
         }
-    // fw_sum over the positions (0, 1, 2) = (m, centre, p) of the neighbourhood along each axis
-    auto A = [&](int x, int y, int z) -> double { return z == 0 ? vm[x][y] : (z == 1 ? v0[x][y] : vp[x][y]); };
-    return fw_sum<T>(A, 0, 1, 2, 0, 1, 2, 0, 1, 2);
+    double s_m = __shfl_up_sync(0xffffffffu, s_p, 1);
+    if (!from_lane) {
+#pragma unroll
+        for (int x = 0; x < 3; x++)
+#pragma unroll
+            for (int y = 0; y < 3; y++) {
+                const double w = (x == 1 ? 2.0 : 1.0) * (y == 1 ? 2.0 : 1.0);
+                // the neighbouring lane's lines: in L1
+                const T m = k > 0 ? ldg(col + X[x] + Y[y] - 1) : pr[x][y][0];
+                if (x == 0 && y == 0) s_m = w * (double)m;
+                else s_m = s_m + w * (double)m;
+            }
+    }
+    T tmp = (T)s_m;
+    tmp = (T)((double)tmp + s_0);
+    tmp = (T)((double)tmp + s_p);
+    return (T)((double)tmp / 64.0);
 }
 
 template <typename T>
