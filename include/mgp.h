@@ -79,7 +79,7 @@ typedef enum { MGP_CYCLE_RELAXATION = 0, MGP_CYCLE_V = 1, MGP_CYCLE_F = 2 } mgp_
                              2 x 85 us) */
 #define MGP_FLAG_FUSED_SETUP 8u /* cycles form the residual inside the restriction kernel (one
                                    launch, r never stored) on every level; without the flag only
-                                   levels of at most 2^20 points do */
+                                   levels of at most 30000 points do */
 
 /* Settings (include/settings.h:14-39) plus the BoundaryCondition and the template choice. */
 typedef struct mgp_desc {

@@ -1039,24 +1039,23 @@ int coarse_setup_fused_t(mgp_solver* s, int l, const FirstSweep<T>& w) {
 // The three-kernel form (large levels): residual (r stored), restriction with u_{l+1} = 0
 // fused, Neumann face restriction.  The one-kernel form leaves r unstored where the residual
 // is formed; nothing reads those values before the next residual overwrites them.
-// Levels of at most kFusedSetupMaxPoints points set up their coarse-grid correction with the
-// one-kernel form: there the two launches it saves outweigh its slower march (on B200, for
-// the 513x257x129 F-cycle: 1.589 ms per iteration with it from 277K-point levels down, 1.635
-// ms without it, 1.719 ms with it from the 2.15M-point level down).  MGP_FLAG_FUSED_SETUP
-// uses it on every level.
-constexpr long long kFusedSetupMaxPoints = 1ll << 20;
+// The one-kernel form is built in only on levels of at most kFusedSetupMaxPoints points, the size
+// up to which visits run in one cluster anyway (so it serves levels kept out of the cluster).
+// Above that the residual and the restriction, now both bound by little more than their launch,
+// are faster apart: with the separate kernels down to 36K points instead of 2^20, on B200 per
+// solve iteration, 161x97x193 576 -> 539 us, 129x65x65 276 -> 246, 65^3 red-black 251 -> 239,
+// 513x257x129 1619 -> 1600, 257x257x129 red-black 1246 -> 1225.  MGP_FLAG_FUSED_SETUP uses the
+// one-kernel form on every level.
+constexpr long long kFusedSetupMaxPoints = 30000;
 
 // The set-up of level l forms its residual in a separate pass (the three-kernel form), which
 // the relaxation before it may take over.
-// FP32 hierarchies use the one-kernel form only up to 2^17 points: the autotuner chose the
-// three-kernel form for their 2^18-point levels (FP32 stencils have half the threads per plane).
 bool setup_residual_separate(const mgp_solver* s, int l) {
     const Geom& G = s->lv[l].G;
     if (s->desc.flags & MGP_FLAG_FUSED_SETUP) return false;
     const int form = s->lv[l].tune[MGP_TUNE_SETUP_FORM];
     if (form) return form == 1;
-    const long long lim = s->dtype == MGP_F32 ? kFusedSetupMaxPoints >> 3 : kFusedSetupMaxPoints;
-    return (long long)G.nx * G.ny * G.nz > lim;
+    return (long long)G.nx * G.ny * G.nz > kFusedSetupMaxPoints;
 }
 
 // resid_done: the relaxation before the set-up already stored r (wavefront pass).
@@ -1217,6 +1216,11 @@ int launch_tail(mgp_solver* s, int t0, bool fcycle, double omega, int64_t ns) {
 }
 
 // ---- the coarse levels in one cluster (mgp_cluster.cuh) -----------------------------------
+// The cluster's finest level has at most kClMaxPoints points: its 16 SMs work a 36K-point level off
+// more slowly than the grid kernels do on all of them (65^3 red-black F-cycle 239 us per iteration
+// with level 1, 36K points, in the cluster and 229 without; 129x65x65 in FP32, 70K points, 276 and
+// 258), while 18.5K points still gain (33x33x17 118 against 128 us).
+constexpr long long kClMaxPoints = kFusedSetupMaxPoints;
 constexpr size_t kClMaxSmem = 216 * 1024;  // dynamic; the argument copy and reduction slots fit beside it
 
 // CTAs of the largest cluster this device co-schedules with that much shared memory: 16 (opt-in
@@ -1359,11 +1363,11 @@ bool cluster_plan(const mgp_solver* s, int t, int nc, ClArgs<T>* a, size_t* smem
     return *smem <= kClMaxSmem;
 }
 
-// First level of the cluster's visits (s->levels: none): the finest level whose hierarchy fits in
-// one cluster's shared memory (about 36K points in FP64).  An operation takes 0.8-1.7 us there
-// against 2.5-3 us as a launch of its own; ten 65^3 red-black F-cycles 3.42 -> 2.56 ms, four FP32
-// 257^3 F-cycles 5.08 -> 4.20 ms, four 33x17x17 F-cycles with their set-up 0.488 -> 0.375 ms.  Not
-// for column-ordered Gauss-Seidel (its sweep runs along x),
+// First level of the cluster's visits (s->levels: none): the finest level of at most kClMaxPoints
+// points whose hierarchy fits in one cluster's shared memory.  An operation takes 0.5-1.5 us there
+// against 2.5-3 us as a launch of its own: without the cluster a solve iteration takes 1588 ->
+// 1645 us on 513x257x129, 229 -> 347 us on 65^3 (red-black), 81 -> 128 us on 33x17x17.  Not for
+// column-ordered Gauss-Seidel (its sweep runs along x),
 // levels with wavefront buffers, or levels whose launch shapes or set-up form were asked for
 // (they are shapes of the per-level kernels), nor beside the one-CTA form.
 int cluster_level(const mgp_solver* s) {
@@ -1371,7 +1375,8 @@ int cluster_level(const mgp_solver* s) {
     const int nc = cluster_ctas(s->device);
     if (!nc) return s->levels;
     for (int l = std::max(0, s->levels - kClMaxLevels); l < s->levels - 1; l++) {
-        bool ok = true;
+        const Geom& G = s->lv[l].G;
+        bool ok = (long long)G.nx * G.ny * G.nz <= kClMaxPoints;
         for (int m = l; m < s->levels && ok; m++) {
             ok = !s->lv[m].gs_column && !s->lv[m].pair;
             for (int p = 0; p < MGP_TUNE_PARAMS; p++) ok = ok && !s->lv[m].tune[p];
