@@ -1591,9 +1591,10 @@ int launch_iteration(mgp_solver* s, int cycle, int64_t ns, double omega) {
     return MGP_OK;
 }
 
-int read_norm(mgp_solver* s, double* out) {
-    // the norm word and, 8 bytes on, the error word of the wavefront passes
-    CK(cudaMemcpyAsync(s->h_norm, s->d_norm, 16, cudaMemcpyDeviceToHost, s->stream));
+// first (may be null): the norm reduced into word 2 before.
+int read_norm(mgp_solver* s, double* out, double* first = nullptr) {
+    // the norm word and, 8 bytes on, the error word of the wavefront and cluster passes
+    CK(cudaMemcpyAsync(s->h_norm, s->d_norm, first ? 24 : 16, cudaMemcpyDeviceToHost, s->stream));
     CK(cudaStreamSynchronize(s->stream));
     if (reinterpret_cast<const int*>(s->h_norm)[2]) {
         CK(cudaMemsetAsync(s->err_word, 0, sizeof(int), s->stream));
@@ -1604,6 +1605,7 @@ int read_norm(mgp_solver* s, double* out) {
     unsigned long long b = *s->h_norm;
     memcpy(&v, &b, sizeof(v));
     *out = v;
+    if (first) memcpy(first, s->h_norm + 2, sizeof(v));
     return MGP_OK;
 }
 
@@ -1870,6 +1872,25 @@ void release(mgp_solver* s) {
     if (s->ev_fork) cudaEventDestroy(s->ev_fork);
     if (s->ev_join) cudaEventDestroy(s->ev_join);
     delete s;
+}
+
+// Dirichlet data of level l into u and u_prev.
+template <typename T>
+int write_faces_t(mgp_solver* s, int l) {
+    LevelState& L = s->lv[l];
+    WriteFacesArgs<T> a{};
+    a.u[0] = (T*)u_ptr(s, l);
+    a.u[1] = L.ubuf[1] ? (T*)uprev_ptr(s, l) : nullptr;
+    a.G = L.G;
+    long long nmax = 0;
+    for (int f = 0; f < 6; f++) {
+        a.g[f] = (const T*)L.face[f];
+        if (s->face_kind[f] != MGP_DIRICHLET) continue;  // Neumann write_to only fills ghosts
+        a.dirichlet |= 1 << f;
+        nmax = std::max(nmax, (long long)(L.face_shape[f][0] * L.face_shape[f][1] * L.face_shape[f][2]));
+    }
+    if (!a.dirichlet) return MGP_OK;
+    return launch_k(s, k_write_faces<T>, dim3((unsigned)grid_1d(s, nmax), 6, a.u[1] ? 2 : 1), dim3(kThreads), 0, a);
 }
 
 struct DeviceGuard {
@@ -2225,21 +2246,7 @@ int mgp_download_face(mgp_solver* s, int face, int l, void* host, int64_t count)
 int mgp_write_bc(mgp_solver* s, int l) {
     CKS(validate_level(s, l));
     DeviceGuard guard(s->device);
-    LevelState& L = s->lv[l];
-    void* targets[2] = {u_ptr(s, l), L.ubuf[1] ? uprev_ptr(s, l) : nullptr};
-    for (void* u : targets) {
-        if (!u) continue;
-        for (int f = 0; f < 6; f++) {  // write_bc_to order: north, south, east, west, top, bottom
-            if (s->face_kind[f] != MGP_DIRICHLET) continue;  // Neumann write_to only fills ghosts
-            const int64_t* fs = L.face_shape[f];
-            const long long n = fs[0] * fs[1] * fs[2];
-            if (s->dtype == MGP_F64)
-                k_write_face<double><<<grid_1d(s, n), kThreads, 0, s->stream>>>((double*)u, L.G, (const double*)L.face[f], f);
-            else
-                k_write_face<float><<<grid_1d(s, n), kThreads, 0, s->stream>>>((float*)u, L.G, (const float*)L.face[f], f);
-            CKS(check_launch(s));
-        }
-    }
+    CKS(DISPATCH(s, (write_faces_t<T>(s, l))));
     CK(cudaStreamSynchronize(s->stream));
     return MGP_OK;
 }
@@ -2695,12 +2702,11 @@ static int solve_refined(mgp_solver* s, int cycle, int64_t ns, double omega, dou
     if (omega < 0) omega = s->desc.relaxation == MGP_JACOBI ? 6.0 / 7.0 : 8.0 / 9.0;
     const int64_t launches_at_start = s->launches + s->inner->launches;
     double fnorm = 0.0, rnorm = 0.0;
-    CK(cudaMemsetAsync(s->d_norm, 0, sizeof(unsigned long long), s->stream));
-    CKS(norm_t<double>(s, s->lv[0].f, 0, s->d_norm));
-    CKS(read_norm(s, &fnorm));
+    CK(cudaMemsetAsync(s->d_norm + 2, 0, sizeof(unsigned long long), s->stream));
+    CKS(norm_t<double>(s, s->lv[0].f, 0, s->d_norm + 2));
     CKS(refine_residual(s, refine_first(s->inner, omega, ns)));
     s->inner->lv[0].first_done = false;  // consumed by the steps' graphs
-    CKS(read_norm(s, &rnorm));
+    CKS(read_norm(s, &rnorm, &fnorm));
     double rel = rnorm / fnorm;
     const double first = rel;
     if (flags & MGP_SOLVE_VERBOSE)
@@ -2752,12 +2758,12 @@ int mgp_solve(mgp_solver* s, int cycle, int64_t nsmooth, double omega, const cha
 
     // initial relative residual (include/libpoisson.h:253-284)
     double fnorm = 0.0, rnorm = 0.0;
+    // (both norms in one read-back: words 0 and 2, word 1 holds the passes' error flag)
     CK(cudaMemsetAsync(s->d_norm, 0, sizeof(unsigned long long), s->stream));
-    CKS(DISPATCH(s, (norm_t<T>(s, s->lv[0].f, 0, s->d_norm))));
-    CKS(read_norm(s, &fnorm));
-    CK(cudaMemsetAsync(s->d_norm, 0, sizeof(unsigned long long), s->stream));
+    CK(cudaMemsetAsync(s->d_norm + 2, 0, sizeof(unsigned long long), s->stream));
+    CKS(DISPATCH(s, (norm_t<T>(s, s->lv[0].f, 0, s->d_norm + 2))));
     CKS(DISPATCH(s, (residual_t<T>(s, 0, s->d_norm))));
-    CKS(read_norm(s, &rnorm));
+    CKS(read_norm(s, &rnorm, &fnorm));
     double rel_res = rnorm / fnorm;
     const double first = rel_res;
     if (verbose) std::cout << std::setw(4) << 0 << ": Initial residual: " << std::setw(8) << rel_res << std::endl;
