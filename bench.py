@@ -48,7 +48,7 @@ E2E_CYCLES = 4
 REF_ARM_CYCLES = 30   # timed cycles of the reference arm (a bounded sample)
 # DRAM bytes (read + write) of one level-0 Jacobi sweep launch at this size, from an ncu capture
 # of the timed launch: ncu --set full --clock-control none --kernel-name-base demangled
-#   -k "regex:k_stencil<double, \(int\)0, \(bool\)0, \(bool\)0>" -s 3 -c 1 python bench.py --kernels --steps 1
+#   -k "regex:k_stencil_planes<double, \(int\)0, \(bool\)0, \(int\)3>" -s 3 -c 1 python bench.py --kernels --steps 1
 # (289.6 MB read + 109.7 MB written; algorithmic 408.2 MB: some of u is still in L2 from the
 # launch before).
 JACOBI_SWEEP_DRAM_BYTES = 399.3e6
@@ -791,7 +791,7 @@ def main():
                    "parallelism": f"replicas x{world}"},
         "e2e": {"value": e2e_value, "unit": UNIT, "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": d2h,
                 "step": f"to_device + {E2E_CYCLES}-cycle solve + to_host", "ms_per_request": 1e3 * e2e_sec},
-        "roofline": {"bound": "hbm", "kernel": "k_stencil<double,OP_JACOBI> level 0", "achieved": achieved,
+        "roofline": {"bound": "hbm", "kernel": "k_stencil_planes<double,OP_JACOBI> level 0", "achieved": achieved,
                      "peak": peak, "unit": "GB/s", "frac": achieved / peak, "peak_kind": peak_kind,
                      "traffic": JACOBI_SWEEP_DRAM_BYTES, "traffic_source": "ncu dram__bytes_read+write, 1 launch",
                      "algorithmic_bytes_per_launch": kbytes, "launch_us": ksec * 1e6},
