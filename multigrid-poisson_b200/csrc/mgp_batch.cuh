@@ -211,6 +211,18 @@ struct BatchProblem {
     int slot = 0;             // norm slot
 };
 
+// The launches of one refinement step of the active problems from one state of the inner
+// hierarchies (which buffer is u on each level): they name buffers, so they are valid from that
+// state only.
+struct BatchSchedule {
+    bool valid = false;
+    std::vector<uint64_t> pre, post;  // inner state bits before and after the step
+    void* d_items = nullptr;
+    size_t d_items_bytes = 0;
+    std::vector<BatchLaunch> launches;
+    cudaGraphExec_t graph = nullptr;
+};
+
 struct mgp_batch {
     mgp_batch_desc desc{};
     int device = 0;
@@ -220,14 +232,12 @@ struct mgp_batch {
     unsigned long long* d_norms = nullptr;  // one slot per problem
     unsigned long long* h_norms = nullptr;
     int slots = 0;
-    // cached schedule of one refinement step for the current active set
+    // Cached schedules of one refinement step for the current active set.  A step either leaves the
+    // state as it found it or swaps the buffers of some levels (Jacobi F-cycles with an odd
+    // number of sweeps), so a steady set of problems alternates between two states at most.
     bool dirty = true;
-    std::vector<uint64_t> sched_state;  // inner state bits the schedule was built from
-    std::vector<uint64_t> post_state;
-    void* d_items = nullptr;
-    size_t d_items_bytes = 0;
-    std::vector<BatchLaunch> launches;
-    cudaGraphExec_t graph = nullptr;
+    BatchSchedule sched[2];
+    int last = 0;  // the schedule of the latest step
     int64_t launches_total = 0;
     int64_t launches_last = 0;  // launches of the latest non-empty schedule
     int stable_steps = 0;       // steps run since the active set last changed
@@ -240,10 +250,14 @@ struct mgp_batch {
 
 namespace {
 
-void batch_free_schedule(mgp_batch* b) {
-    if (b->graph) cudaGraphExecDestroy(b->graph);
-    b->graph = nullptr;
-    b->launches.clear();
+void batch_free_schedule(BatchSchedule& q) {
+    if (q.graph) cudaGraphExecDestroy(q.graph);
+    q.graph = nullptr;
+    q.launches.clear();
+    q.valid = false;
+}
+void batch_free_schedules(mgp_batch* b) {
+    for (auto& q : b->sched) batch_free_schedule(q);
 }
 
 // The first sweep that the refinement residual of a problem writes for the step after it.
@@ -443,35 +457,40 @@ int build_step(mgp_batch* b, ScheduleBuilder& sb) {
 
 int batch_inner_dtype(const mgp_batch* b) { return b->desc.inner_dtype; }
 
-int batch_rebuild(mgp_batch* b) {
-    batch_free_schedule(b);
+// Inner state bits of every problem, the key of a schedule.
+std::vector<uint64_t> batch_state(const mgp_batch* b) {
+    std::vector<uint64_t> v;
+    for (auto& p : b->probs) v.push_back(p.s ? state_bits(p.s->inner) : 0);
+    return v;
+}
+
+// Builds q for the present state.
+int batch_build(mgp_batch* b, BatchSchedule& q) {
+    batch_free_schedule(q);
     // record each active problem's inner state, build (this advances it), note the post
-    // state and restore: the graph launch applies the post state
-    std::vector<uint64_t> pre;
-    for (auto& p : b->probs) pre.push_back(p.s ? state_bits(p.s->inner) : 0);
+    // state and restore: the step applies the post state
+    const std::vector<uint64_t> pre = batch_state(b);
     ScheduleBuilder sb;
     sb.sms = sm_count(b->device);
     int st = batch_inner_dtype(b) == MGP_F32 ? build_step<float>(b, sb) : build_step<double>(b, sb);
-    b->post_state.clear();
-    for (size_t i = 0; i < b->probs.size(); i++) {
-        b->post_state.push_back(b->probs[i].s ? state_bits(b->probs[i].s->inner) : 0);
+    q.post = batch_state(b);
+    for (size_t i = 0; i < b->probs.size(); i++)
         if (b->probs[i].s) set_state_bits(b->probs[i].s->inner, pre[i]);
-    }
-    b->sched_state = pre;
+    q.pre = pre;
     if (st != MGP_OK) return st;
-    if (sb.bytes.size() > b->d_items_bytes) {
-        if (b->d_items) cudaFree(b->d_items);
-        b->d_items = nullptr;
-        b->d_items_bytes = 0;
-        CK(cudaMalloc(&b->d_items, sb.bytes.size()));
-        b->d_items_bytes = sb.bytes.size();
+    if (sb.bytes.size() > q.d_items_bytes) {
+        if (q.d_items) cudaFree(q.d_items);
+        q.d_items = nullptr;
+        q.d_items_bytes = 0;
+        CK(cudaMalloc(&q.d_items, sb.bytes.size()));
+        q.d_items_bytes = sb.bytes.size();
     }
     if (!sb.bytes.empty())
-        CK(cudaMemcpyAsync(b->d_items, sb.bytes.data(), sb.bytes.size(), cudaMemcpyHostToDevice, b->stream));
+        CK(cudaMemcpyAsync(q.d_items, sb.bytes.data(), sb.bytes.size(), cudaMemcpyHostToDevice, b->stream));
     CK(cudaStreamSynchronize(b->stream));
-    b->launches = sb.launches;
-    if (!b->launches.empty()) b->launches_last = (int64_t)b->launches.size();
-    b->dirty = false;
+    q.launches = sb.launches;
+    if (!q.launches.empty()) b->launches_last = (int64_t)q.launches.size();
+    q.valid = true;
     return MGP_OK;
 }
 
@@ -479,20 +498,20 @@ int batch_rebuild(mgp_batch* b) {
 // set changed run this way (capturing and instantiating a graph of a few hundred launches
 // costs more than launching them a few times; the host issues them while the GPU works).
 constexpr int kBatchCaptureAfter = 3;
-int batch_launch_direct(mgp_batch* b) {
+int batch_launch_direct(mgp_batch* b, const BatchSchedule& q) {
     CK(cudaMemsetAsync(b->d_norms, 0, sizeof(unsigned long long) * b->slots, b->stream));
-    for (auto& L : b->launches) L.fn((const char*)b->d_items + L.offset, L.n, L.total, L.grid, b->stream);
+    for (auto& L : q.launches) L.fn((const char*)q.d_items + L.offset, L.n, L.total, L.grid, b->stream);
     CK(cudaGetLastError());
     return MGP_OK;
 }
 
-// Capture of the current schedule, replayed every step while the active set stays the same.
-int batch_capture(mgp_batch* b) {
+// Capture of a schedule, replayed by every step from its state while the active set stays the same.
+int batch_capture(mgp_batch* b, BatchSchedule& q) {
     cudaGraph_t g = nullptr;
     CK(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
     // the step's last launch max-reduces each problem's residual into its slot
     cudaError_t me = cudaMemsetAsync(b->d_norms, 0, sizeof(unsigned long long) * b->slots, b->stream);
-    for (auto& L : b->launches) L.fn((const char*)b->d_items + L.offset, L.n, L.total, L.grid, b->stream);
+    for (auto& L : q.launches) L.fn((const char*)q.d_items + L.offset, L.n, L.total, L.grid, b->stream);
     if (me != cudaSuccess) {
         cudaGraph_t g0 = nullptr;
         cudaStreamEndCapture(b->stream, &g0);
@@ -505,10 +524,10 @@ int batch_capture(mgp_batch* b) {
         if (g) cudaGraphDestroy(g);
         return fail(MGP_ERR_CUDA, "batch graph capture: %s", cudaGetErrorString(le != cudaSuccess ? le : e));
     }
-    cudaError_t ei = cudaGraphInstantiate(&b->graph, g, 0);
+    cudaError_t ei = cudaGraphInstantiate(&q.graph, g, 0);
     cudaGraphDestroy(g);
     if (ei != cudaSuccess) {
-        b->graph = nullptr;
+        q.graph = nullptr;
         return fail(MGP_ERR_CUDA, "batch graph instantiate: %s", cudaGetErrorString(ei));
     }
     return MGP_OK;
@@ -614,12 +633,13 @@ int mgp_batch_destroy(mgp_batch* b) {
     if (!b) return MGP_OK;
     DeviceGuard guard(b->device);
     cudaStreamSynchronize(b->stream);
-    batch_free_schedule(b);
+    batch_free_schedules(b);
     for (auto& p : b->probs)
         if (p.s) mgp_destroy(p.s);
     cudaStreamSynchronize(b->stream);  // the problems' memory is back in the pool
     if (b->pool) cudaMemPoolDestroy(b->pool);
-    if (b->d_items) cudaFree(b->d_items);
+    for (auto& q : b->sched)
+        if (q.d_items) cudaFree(q.d_items);
     if (b->d_norms) cudaFree(b->d_norms);
     if (b->h_norms) cudaFreeHost(b->h_norms);
     if (b->h_slab) cudaFreeHost(b->h_slab);
@@ -704,7 +724,7 @@ int mgp_batch_remove(mgp_batch* b, int id) {
     if (!p) return fail(MGP_ERR_INVALID_ARG, "no problem %d in the batch", id);
     DeviceGuard guard(b->device);
     cudaStreamSynchronize(b->stream);
-    batch_free_schedule(b);  // the graph refers to this problem's buffers
+    batch_free_schedules(b);  // their graphs refer to this problem's buffers
     mgp_destroy(p->s);
     p->s = nullptr;
     p->active = false;
@@ -725,37 +745,44 @@ int mgp_batch_step(mgp_batch* b, int* n_active) {
     if (!b) return fail(MGP_ERR_INVALID_ARG, "null batch");
     DeviceGuard guard(b->device);
     CKS(batch_start_new(b));
-    std::vector<uint64_t> cur;
-    for (auto& p : b->probs) cur.push_back(p.s ? state_bits(p.s->inner) : 0);
-    const bool changed = b->dirty || cur != b->sched_state;
-    if (changed) {
-        CKS(batch_rebuild(b));  // schedule only
+    if (b->dirty) {
+        batch_free_schedules(b);
         b->stable_steps = 0;
-    } else if (!b->graph && !b->launches.empty() && b->stable_steps >= kBatchCaptureAfter) {
-        CKS(batch_capture(b));  // the set has held for a while: replay it as a graph
     }
+    // the schedule of the present state; else one is built, in the place of the one not used last
+    const std::vector<uint64_t> cur = batch_state(b);
+    int at = -1;
+    for (int k = 0; k < 2; k++)
+        if (b->sched[k].valid && b->sched[k].pre == cur) at = k;
+    if (at < 0) {
+        at = b->sched[b->last].valid ? 1 - b->last : b->last;
+        CKS(batch_build(b, b->sched[at]));
+        b->dirty = false;
+    } else if (!b->sched[at].graph && !b->sched[at].launches.empty() && b->stable_steps >= kBatchCaptureAfter) {
+        CKS(batch_capture(b, b->sched[at]));  // the set has held for a while: replay it as a graph
+    }
+    b->last = at;
+    const BatchSchedule& q = b->sched[at];
     b->stable_steps++;
     int n = 0;
     for (auto& p : b->probs) n += (p.s && p.active && p.started);
     if (n_active) *n_active = n;
-    if (!n || b->launches.empty()) return MGP_OK;
-    if (b->graph) CK(cudaGraphLaunch(b->graph, b->stream));
-    else CKS(batch_launch_direct(b));
-    b->launches_total += (int64_t)b->launches.size();
+    if (!n || q.launches.empty()) return MGP_OK;
+    if (q.graph) CK(cudaGraphLaunch(q.graph, b->stream));
+    else CKS(batch_launch_direct(b, q));
+    b->launches_total += (int64_t)q.launches.size();
     CK(cudaMemcpyAsync(b->h_norms, b->d_norms, sizeof(unsigned long long) * b->slots, cudaMemcpyDeviceToHost, b->stream));
     CK(cudaStreamSynchronize(b->stream));
     for (size_t i = 0; i < b->probs.size(); i++) {
         BatchProblem& p = b->probs[i];
         if (!p.s) continue;
-        set_state_bits(p.s->inner, b->post_state[i]);
+        set_state_bits(p.s->inner, q.post[i]);
         if (!p.active || !p.started) continue;
         double rn;
         memcpy(&rn, b->h_norms + p.slot, 8);
         p.rel = rn / p.fnorm;
         p.iters++;
     }
-    b->sched_state.clear();
-    for (auto& p : b->probs) b->sched_state.push_back(p.s ? state_bits(p.s->inner) : 0);
     return MGP_OK;
 }
 
@@ -812,7 +839,8 @@ int mgp_batch_solve(mgp_batch* b, double tol, int64_t maxiter, int64_t* steps) {
 
 int mgp_batch_kernel_launches(const mgp_batch* b, int64_t* per_step) {
     if (!b || !per_step) return fail(MGP_ERR_INVALID_ARG, "null argument");
-    *per_step = b->launches.empty() ? b->launches_last : (int64_t)b->launches.size();
+    const auto& launches = b->sched[b->last].launches;
+    *per_step = launches.empty() ? b->launches_last : (int64_t)launches.size();
     return MGP_OK;
 }
 
