@@ -540,11 +540,20 @@ BatchProblem* batch_find(mgp_batch* b, int id) {
 }
 
 // f norm and first FP64 residual of problems that have not started (their data is on the
-// device now); each is its own small launch on the batch stream.
+// device now); each is its own small launch on the batch stream.  A started problem whose next
+// correction was begun with other smoothing than the batch's (it was solved on its own between
+// two steps) has it begun again from its present residual.
 int batch_start_new(mgp_batch* b) {
     bool any = false;
     for (auto& p : b->probs) {
-        if (!p.s || p.started || !p.active) continue;
+        if (!p.s || !p.active) continue;
+        if (p.started) {
+            const RefineFirst w = batch_first(b, p.s->inner);
+            if (p.s->inner->guess == w) continue;
+            CKS(refine_residual(p.s, w));
+            p.s->inner->lv[0].first_done = false;  // build_step knows
+            continue;
+        }
         mgp_solver* s = p.s;
         std::swap(s->stream, b->stream);  // issue on the batch stream
         unsigned long long* saved = s->d_norm;
@@ -778,6 +787,7 @@ int mgp_batch_step(mgp_batch* b, int* n_active) {
         if (!p.s) continue;
         set_state_bits(p.s->inner, q.post[i]);
         if (!p.active || !p.started) continue;
+        p.s->inner->guess = batch_first(b, p.s->inner);
         double rn;
         memcpy(&rn, b->h_norms + p.slot, 8);
         p.rel = rn / p.fnorm;

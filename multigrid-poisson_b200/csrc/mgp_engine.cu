@@ -116,6 +116,14 @@ struct GraphEntry {
     int64_t kernels = 0;  // kernel nodes in the graph
 };
 
+// The first sweep of a correction's zero guess that the refinement residual writes along
+// (RefineArgs::first): the smoothing of the correction cycle that follows.
+struct RefineFirst {
+    int on = 0;  // 0 none, 1 Jacobi, 2 red-black
+    double omega = 0;
+    bool operator==(const RefineFirst& o) const { return on == o.on && (!on || omega == o.omega); }
+};
+
 struct mgp_solver {
     mgp_desc desc{};
     int dtype = MGP_F64;
@@ -138,6 +146,7 @@ struct mgp_solver {
     // `inner` the correction hierarchy (all levels, FP32 or FP64, zero boundary data).  The
     // inner solver shares this solver's stream.
     mgp_solver* inner = nullptr;
+    RefineFirst guess;  // inner solvers: the sweep that level 0's guess holds
     bool owns_stream = true;
     // Side stream of the coarse-grid set-up: the Neumann face restriction runs on it, forked
     // and joined by the two events, overlapped with the residual (own-memory solvers only).
@@ -1610,12 +1619,7 @@ int read_norm(mgp_solver* s, double* out, double* first = nullptr) {
 }
 
 // ---- iterative refinement ------------------------------------------------------------
-// The inner first sweep that the refinement residual writes along (RefineArgs::first): the
-// smoothing of the correction cycle that follows.
-struct RefineFirst {
-    int on = 0;  // 0 none, 1 Jacobi, 2 red-black
-    double omega = 0;
-};
+// The first sweep of the corrections of (omega, ns).
 RefineFirst refine_first(const mgp_solver* in, double omega, int64_t ns) {
     RefineFirst w;
     if (ns >= 1 && !in->lv[0].gs_column && !in->lv[0].wave) w.on = in->desc.relaxation == MGP_JACOBI ? 1 : 2;
@@ -1667,7 +1671,10 @@ int refine_residual_t(mgp_solver* s, const RefineFirst& w) {
     chunks = (L.G.nx + a.ichunk - 1) / a.ichunk;
     CK(cudaMemsetAsync(s->d_norm, 0, sizeof(unsigned long long), s->stream));
     CKS(launch_k(s, k_refine_residual<double, Ti, R>, dim3(bx, chunks), dim3(kThreads), 0, a));
-    if (!R) s->inner->lv[0].first_done = w.on != 0;
+    if (!R) {
+        s->inner->lv[0].first_done = w.on != 0;
+        s->inner->guess = w;
+    }
     return MGP_OK;
 }
 
@@ -1700,10 +1707,10 @@ int launch_refine_step(mgp_solver* s, int cycle, int64_t ns, double omega) {
     memcpy(&ob, &omega, sizeof(ob));
     auto key = std::make_tuple(100 + cycle, ns, ob, state_bits(in));
     auto it = s->graphs.find(key);
+    const RefineFirst w = refine_first(in, omega, ns);
     if (it == s->graphs.end()) {
         const uint64_t pre = state_bits(in);
         const int64_t s0 = s->launches, i0 = in->launches;
-        const RefineFirst w = refine_first(in, omega, ns);
         in->lv[0].first_done = w.on != 0;  // the residual before this step wrote the first sweep
         cudaGraph_t g = nullptr;
         CK(cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal));
@@ -1735,6 +1742,7 @@ int launch_refine_step(mgp_solver* s, int cycle, int64_t ns, double omega) {
     }
     CK(cudaGraphLaunch(it->second.exec, s->stream));
     set_state_bits(in, it->second.post_state);
+    in->guess = w;
     s->launches += it->second.kernels;
     return MGP_OK;
 }
