@@ -601,6 +601,7 @@ int launch_wave(mgp_solver* s, int l, int nj, int res, bool wu1, T omega, unsign
 #define MGP_SHORT_MARCH 1  // compile-time switch of the short-march rule in launch_stencil
 #endif
 constexpr long long kShortMarchMinPoints = 1ll << 22;
+constexpr int kMaxGridRows = 65535;  // largest gridDim.y: boxes of more chunks keep the long march
 
 // Large levels whose plane does not fill a wave of blocks march short chunks.  Measured on B200
 // with the autotuner (F-cycles on 513x257x129 and 257^3): 3-5 planes per block were fastest in
@@ -612,7 +613,7 @@ template <typename T>
 int short_march_chunks(const Geom& G, int bx, int cap, int chunks) {
     constexpr int kShort = sizeof(T) == 8 ? 4 : 3;
     if (MGP_SHORT_MARCH && bx < cap && (long long)G.nx * G.ny * G.nz >= kShortMarchMinPoints &&
-        (G.nx + chunks - 1) / chunks > kShort)
+        (G.nx + chunks - 1) / chunks > kShort && (G.nx + kShort - 1) / kShort <= kMaxGridRows)
         return (G.nx + kShort - 1) / kShort;
     return chunks;
 }
@@ -629,10 +630,11 @@ int short_march_chunks(const Geom& G, int bx, int cap, int chunks) {
 template <typename T, int OP>
 int planes_in_registers(const Geom& G, int ichunk, bool built_in) {
     if (!built_in || ichunk == 1) return 0;
-    if ((long long)G.nx * G.ny * G.nz < kShortMarchMinPoints) return 2;
+    auto fits = [&](int P) { return (G.nx + P - 1) / P <= kMaxGridRows ? P : 0; };
+    if ((long long)G.nx * G.ny * G.nz < kShortMarchMinPoints) return fits(2);
     constexpr int kShort = sizeof(T) == 8 ? 4 : 3;
     if (ichunk > kShort || (OP == OP_RESIDUAL && sizeof(T) == 8)) return 0;
-    return 3;
+    return fits(3);
 }
 
 template <typename T, int OP>
