@@ -206,8 +206,9 @@ int mgp_relax(mgp_solver* s, int level, double omega, int64_t nsmooth);
  * colours themselves: a domain split into slabs exchanges its halo planes between the two
  * half-sweeps.  UNSUPPORTED for Jacobi solvers. */
 int mgp_relax_colour(mgp_solver* s, int level, double omega, int colour);
-/* Failure detection of the wavefront passes (MGP_FLAG_WAVE): bound on the polls of a wait for a
- * plane copy (0 = the default, 2^22).  A wait that runs out marks the pass failed; the pass
+/* Failure detection of the wavefront passes (MGP_FLAG_WAVE) and of the coarse levels that run in one
+ * thread-block cluster: bound on the polls of a wait for a plane copy, or for a neighbouring
+ * CTA's planes (0 = the default, 2^22).  A wait that runs out marks the pass failed; the pass
  * still lets every copy it issued land before it exits, and the next norm read-back (the solve
  * loop's) returns MGP_ERR_TIMEOUT.  No counterpart in the reference (its target regions are
  * synchronous); a test sets a bound of 1 to drive the failure path without a GPU fault. */

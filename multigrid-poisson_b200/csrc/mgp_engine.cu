@@ -157,7 +157,7 @@ struct mgp_solver {
     // batch's pinned slab.
     cudaMemPool_t pool = nullptr;
     bool owns_h_norm = true;
-    unsigned wait_polls = kWaitPolls;  // bound of the wavefront passes' waits for a copy
+    unsigned wait_polls = kWaitPolls;  // bound of the wavefront passes' and the cluster's waits
 };
 
 // Where a solver's memory comes from: nullptr = its own stream, cudaMalloc, pinned read-back.
@@ -1418,6 +1418,7 @@ int launch_cluster(mgp_solver* s, int t, bool f, bool v, double omega, int64_t n
     a.alt = s->gs_alternate;
     a.norm = norm;
     a.err = s->err_word;
+    a.polls = s->wait_polls;
     for (int m = 0; m < a.nl; m++) {
         LevelState& L = s->lv[t + m];
         ClLevel<T>& q = a.L[m];
@@ -1607,10 +1608,12 @@ int read_norm(mgp_solver* s, double* out, double* first = nullptr) {
     // the norm word and, 8 bytes on, the error word of the wavefront and cluster passes
     CK(cudaMemcpyAsync(s->h_norm, s->d_norm, first ? 24 : 16, cudaMemcpyDeviceToHost, s->stream));
     CK(cudaStreamSynchronize(s->stream));
-    if (reinterpret_cast<const int*>(s->h_norm)[2]) {
+    if (const int err = reinterpret_cast<const int*>(s->h_norm)[2]) {
         CK(cudaMemsetAsync(s->err_word, 0, sizeof(int), s->stream));
         CK(cudaStreamSynchronize(s->stream));
-        return fail(MGP_ERR_TIMEOUT, "wavefront pass: a shared-memory ring wait ran out of time; results are invalid");
+        return fail(MGP_ERR_TIMEOUT, "%s; results are invalid",
+                    err == kErrCluster ? "coarse levels in a cluster: a wait for a neighbour's planes ran out"
+                                       : "wavefront pass: a shared-memory ring wait ran out of time");
     }
     double v;
     unsigned long long b = *s->h_norm;
