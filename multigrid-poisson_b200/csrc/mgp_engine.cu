@@ -148,8 +148,8 @@ struct mgp_solver {
     mgp_solver* inner = nullptr;
     RefineFirst guess;  // inner solvers: the sweep that level 0's guess holds
     bool owns_stream = true;
-    // Side stream of the coarse-grid set-up: the Neumann face restriction runs on it, forked
-    // and joined by the two events, overlapped with the residual (own-memory solvers only).
+    // Side stream of the coarse-grid set-up on large levels: the Neumann face restriction runs on
+    // it, forked and joined by the two events, overlapped with the residual (own-memory solvers only).
     cudaStream_t side = nullptr;
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
     // Problems of a batch allocate from the batch's memory pool in the batch's stream order
@@ -637,8 +637,9 @@ int planes_in_registers(const Geom& G, int ichunk, bool built_in) {
     return fits(3);
 }
 
-template <typename T, int OP>
-int launch_stencil(mgp_solver* s, int l, const void* src, void* dst, T omega, int colour, unsigned long long* norm) {
+// Arguments of a stencil over level l, but for the planes per block.
+template <typename T>
+StencilArgs<T> level_stencil(mgp_solver* s, int l, const void* src, void* dst, T omega, int colour, unsigned long long* norm) {
     LevelState& L = s->lv[l];
     StencilArgs<T> a;
     a.G = L.G;
@@ -655,43 +656,66 @@ int launch_stencil(mgp_solver* s, int l, const void* src, void* dst, T omega, in
     hsq_terms(a.hsq, a.inv_hsq, a.hsq_pow2);
     a.colour = colour;
     a.norm = norm;
+    return a;
+}
+
+// How a stencil over level l is cut: bx blocks cover a plane, `chunks` of `ichunk` planes; regs: in
+// the register form (k_stencil_planes), else the march.
+struct StencilShape {
+    int bx = 1, chunks = 1, ichunk = 1;
+    bool regs = false;
+    dim3 grid() const { return dim3(bx, chunks); }
+};
+template <typename T, int OP>
+StencilShape stencil_shape(mgp_solver* s, int l, bool norm) {
+    LevelState& L = s->lv[l];
     constexpr int V = VecT<T>::V;
+    StencilShape q;
     const int plane = L.G.ny * ((L.G.nz + V - 1) / V);  // threads per plane
-    const int bx = (plane + kThreads - 1) / kThreads;
-    int chunks = 1;
+    q.bx = (plane + kThreads - 1) / kThreads;
     bool built_in = true;
-    if (OP != OP_GS_COLUMN) {
+    if constexpr (OP != OP_GS_COLUMN) {
         const bool nrm = OP == OP_RESIDUAL && norm;
         const int planes = L.tune[OP == OP_RESIDUAL ? (nrm ? MGP_TUNE_NORM_PLANES : MGP_TUNE_RESID_PLANES)
                                                     : MGP_TUNE_RELAX_PLANES];
         if (planes > 0) {
-            chunks = (L.G.nx + planes - 1) / planes;
+            q.chunks = (L.G.nx + planes - 1) / planes;
             built_in = false;
         } else {
             const int cap = sm_count(s->device) *
                             (nrm ? (std::is_same<T, double>::value ? resident_blocks(k_residual_norm64<false>)
                                                                     : resident_blocks(k_stencil<T, OP, true>))
                                  : resident_blocks(k_stencil<T, OP, false>));
-            chunks = march_chunks(bx, L.G.nx, cap);
-            chunks = short_march_chunks<T>(L.G, bx, cap, chunks);
+            q.chunks = march_chunks(q.bx, L.G.nx, cap);
+            q.chunks = short_march_chunks<T>(L.G, q.bx, cap, q.chunks);
         }
     }
-    a.ichunk = (L.G.nx + chunks - 1) / chunks;
-    chunks = (L.G.nx + a.ichunk - 1) / a.ichunk;
-    dim3 grid(bx, chunks);
+    q.ichunk = (L.G.nx + q.chunks - 1) / q.chunks;
     if constexpr (OP != OP_GS_COLUMN) {
-        const int P = planes_in_registers<T, OP>(L.G, a.ichunk, built_in);
-        if (P) {
-            a.ichunk = P;
-            const dim3 g(bx, (L.G.nx + P - 1) / P);
+        const int P = planes_in_registers<T, OP>(L.G, q.ichunk, built_in);
+        q.regs = P != 0;
+        if (P) q.ichunk = P;
+    }
+    q.chunks = (L.G.nx + q.ichunk - 1) / q.ichunk;
+    return q;
+}
+
+template <typename T, int OP>
+int launch_stencil(mgp_solver* s, int l, const void* src, void* dst, T omega, int colour, unsigned long long* norm) {
+    const StencilShape q = stencil_shape<T, OP>(s, l, norm != nullptr);
+    StencilArgs<T> a = level_stencil<T>(s, l, src, dst, omega, colour, norm);
+    a.ichunk = q.ichunk;
+    const dim3 grid = q.grid();
+    if constexpr (OP != OP_GS_COLUMN) {
+        if (q.regs) {
             if constexpr (OP == OP_RESIDUAL) {
-                if (norm && P == 2) return launch_k(s, k_stencil_planes<T, OP, true, 2>, g, dim3(kThreads), 0, a);
+                if (norm && q.ichunk == 2) return launch_k(s, k_stencil_planes<T, OP, true, 2>, grid, dim3(kThreads), 0, a);
                 if constexpr (std::is_same<T, float>::value)
-                    if (norm) return launch_k(s, k_stencil_planes<T, OP, true, 3>, g, dim3(kThreads), 0, a);
+                    if (norm) return launch_k(s, k_stencil_planes<T, OP, true, 3>, grid, dim3(kThreads), 0, a);
             }
-            if (P == 2) return launch_k(s, k_stencil_planes<T, OP, false, 2>, g, dim3(kThreads), 0, a);
+            if (q.ichunk == 2) return launch_k(s, k_stencil_planes<T, OP, false, 2>, grid, dim3(kThreads), 0, a);
             if constexpr (!(OP == OP_RESIDUAL && std::is_same<T, double>::value))
-                return launch_k(s, k_stencil_planes<T, OP, false, 3>, g, dim3(kThreads), 0, a);
+                return launch_k(s, k_stencil_planes<T, OP, false, 3>, grid, dim3(kThreads), 0, a);
         }
     }
     if constexpr (std::is_same<T, double>::value && OP == OP_RESIDUAL) {
@@ -1069,6 +1093,41 @@ bool setup_residual_separate(const mgp_solver* s, int l) {
     return (long long)G.nx * G.ny * G.nz > kFusedSetupMaxPoints;
 }
 
+// The residual of level l and the Neumann face restriction to level l+1 in one launch, where the
+// residual takes its built-in shape on levels below kFacesMaxPoints (*done tells).  The side
+// stream adds a branch to the captured graph at every visit, which the first solve of a solver
+// pays for (capture and instantiation), Neumann face or not; on B200, four iterations (three on
+// 257x129x65), with the side stream on every level above 30000 points, and now: 161x97x193 3.81 ->
+// 2.76 ms, 257x129x65 1.87 -> 1.33, 513x257x129 F 6.83 -> 6.17 and V 3.38 -> 3.20 (6.34 and 3.26
+// with the limit at 2^20), 65^3 all Dirichlet 2.92 -> 2.50; later solves take the same time.
+// Above the limit the residual is a march of its own and the side stream stays.
+constexpr long long kFacesMaxPoints = kShortMarchMinPoints;
+template <typename T>
+int residual_faces_t(mgp_solver* s, int l, bool* done) {
+    *done = false;
+    const Geom& G = s->lv[l].G;
+    if ((long long)G.nx * G.ny * G.nz >= kFacesMaxPoints) return MGP_OK;
+    const StencilShape q = stencil_shape<T, OP_RESIDUAL>(s, l, false);
+    if (!(q.regs && q.ichunk == 2) && !(q.ichunk == 1 && !s->lv[l].tune[MGP_TUNE_RESID_PLANES])) return MGP_OK;
+    ResidualFacesArgs<T> a;
+    bool any = false;
+    a.s = level_stencil<T>(s, l, u_ptr(s, l), s->lv[l].r, T(0), 0, nullptr);
+    a.s.ichunk = q.ichunk;
+    a.bc = bc_args<T>(s, l, &any);
+    long long nmax = 1;
+    for (int f = 0; f < 6; f++) {
+        const int64_t* fs = s->lv[l + 1].face_shape[f];
+        nmax = std::max(nmax, (long long)(fs[0] * fs[1] * fs[2]));
+    }
+    a.per_face = (int)((nmax + kThreads - 1) / kThreads);
+    a.rows = (6 * a.per_face + q.bx - 1) / q.bx;
+    if (q.chunks + a.rows > kMaxGridRows) return MGP_OK;
+    *done = true;
+    const dim3 grid(q.bx, q.chunks + a.rows);
+    if (q.regs) return launch_k(s, k_residual_faces<T, 2>, grid, dim3(kThreads), 0, a);
+    return launch_k(s, k_residual_faces<T, 1>, grid, dim3(kThreads), 0, a);
+}
+
 // resid_done: the relaxation before the set-up already stored r (wavefront pass).
 template <typename T>
 int coarse_setup_t(mgp_solver* s, int l, double omega, int64_t ns, bool resid_done = false) {
@@ -1077,9 +1136,15 @@ int coarse_setup_t(mgp_solver* s, int l, double omega, int64_t ns, bool resid_do
         CKS(coarse_setup_fused_t<T>(s, l, w));
     } else {
         // The face restriction (reads u and the fine faces) and the residual (reads u, writes r)
-        // are independent: the face restriction runs on the side stream meanwhile, joined before
-        // the restriction, whose first coarse sweep reads the coarse faces.
-        if (!resid_done && s->side) {
+        // are independent: the face restriction runs in blocks of the residual's launch or, beside
+        // longer ones, on the side stream, joined before the restriction, whose first coarse sweep
+        // reads the coarse faces.
+        bool any = false, done = false;
+        for (int f = 0; f < 6; f++) any = any || s->face_kind[f] == MGP_NEUMANN;
+        if (any && !resid_done) CKS(residual_faces_t<T>(s, l, &done));
+        if (done) {
+            // r and the coarse faces are there
+        } else if (any && !resid_done && s->side) {
             CK(cudaEventRecord(s->ev_fork, s->stream));
             CK(cudaStreamWaitEvent(s->side, s->ev_fork, 0));
             CKS(restrict_bc_t<T>(s, l, s->side));

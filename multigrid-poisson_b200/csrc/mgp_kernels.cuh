@@ -970,6 +970,31 @@ __global__ void __launch_bounds__(256) k_restrict_bc(BcRestrictArgs<T> a) {
     bc_restrict_tile(a, blockIdx.x, blockIdx.y, gridDim.x);
 }
 
+// The residual of a level and the Neumann face restriction to the next one, both of which only
+// read u and the fine faces, in one launch: the first `rows` rows of the grid restrict the
+// faces (`per_face` blocks each; few points in long chains, so they start first), the others
+// form the residual, P planes per block as k_stencil_planes, or one (P = 1).
+template <typename T>
+struct ResidualFacesArgs {
+    StencilArgs<T> s;
+    BcRestrictArgs<T> bc;
+    int per_face, rows;
+};
+
+template <typename T, int P>
+__global__ void __launch_bounds__(256, 4) k_residual_faces(const __grid_constant__ ResidualFacesArgs<T> a) {
+    pdl_begin();
+    const int by = (int)blockIdx.y - a.rows;
+    if (by < 0) {
+        const int b = blockIdx.y * gridDim.x + blockIdx.x;
+        if (b < 6 * a.per_face) bc_restrict_tile(a.bc, b % a.per_face, b / a.per_face, a.per_face);
+    } else if (P == 1) {
+        stencil_tile<T, OP_RESIDUAL, false, true>(a.s, blockIdx.x, by);
+    } else {
+        stencil_planes<T, OP_RESIDUAL, false, P>(a.s, blockIdx.x, by);
+    }
+}
+
 // ------------------------------------------------------------------------------------
 // Coarse-grid set-up in one pass (include/vcycle.h:34-76): the residual of level l is
 // formed plane by plane and never stored, restricted into f_{l+1} (Injection or
