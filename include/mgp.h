@@ -78,8 +78,9 @@ typedef enum { MGP_CYCLE_RELAXATION = 0, MGP_CYCLE_V = 1, MGP_CYCLE_F = 2 } mgp_
                              than the separate passes (513x257x129 FP64: two sweeps 234 us against
                              2 x 85 us) */
 #define MGP_FLAG_FUSED_SETUP 8u /* cycles form the residual inside the restriction kernel (one
-                                   launch, r never stored) on every level; without the flag only
-                                   levels of at most 30000 points do */
+                                   launch, r never stored) on every level, and no level runs in a
+                                   cluster; without the flag only levels of at most 30000 points that
+                                   are kept out of the cluster do */
 
 /* Settings (include/settings.h:14-39) plus the BoundaryCondition and the template choice. */
 typedef struct mgp_desc {
@@ -242,7 +243,10 @@ int mgp_norm(mgp_solver* s, int field, int level, double* out);
 /* ---- launch-shape tuning (no counterpart in the reference, whose OpenMP target regions
  * take the runtime's teams) ----
  * Per level: how the kernels of that level cut their work.  None of these changes any
- * value a kernel computes or the order of its arithmetic: results stay bit-identical. */
+ * value a kernel computes or the order of its arithmetic: results stay bit-identical.
+ * By default the levels of at most 30000 points whose fields fit there run in one thread-block
+ * cluster, one launch per visit of the cycle.  The parameters shape the per-level kernels, so any
+ * value other than 0 on a level keeps it and every finer level out of the cluster. */
 #define MGP_TUNE_RELAX_PLANES 0 /* planes marched per block by the relaxation (0 = built-in choice) */
 #define MGP_TUNE_RESID_PLANES 1 /* planes per block of the residual */
 #define MGP_TUNE_NORM_PLANES 2  /* planes per block of the residual + max-norm (solve loop) */
@@ -250,8 +254,8 @@ int mgp_norm(mgp_solver* s, int field, int level, double* out);
 #define MGP_TUNE_SETUP_PLANES 4 /* coarse planes per block of the one-kernel set-up (0 = built-in) */
 #define MGP_TUNE_WAVE 5         /* 0 built-in (wavefront passes where MGP_FLAG_WAVE prepared them), 1 off */
 #define MGP_TUNE_TAIL 6         /* level 0 only: 1 runs each cycle visit of the coarsest levels that fit in one
-                                   CTA's shared memory as one launch of one block; 0 (built-in) keeps the
-                                   grid kernels, which are faster on B200 for the 513x257x129 hierarchy */
+                                   CTA's shared memory as one launch of one block, and no level in a
+                                   cluster; 0 (built-in) leaves them to the cluster, which is faster */
 #define MGP_TUNE_PROLONG_SWEEP 7 /* prolongation + add fused with the first Jacobi sweep after it (levels >= 1,
                                     nsmooth even): 0 built-in (levels of at most 2^16 points), 1 separate
                                     passes, 2 fused */
@@ -264,8 +268,9 @@ int mgp_get_tuning(mgp_solver* s, int level, int param, int64_t* value);
  * with CUDA events -- and keeps them on the solver.  Refinement solvers tune their correction
  * hierarchy.  Every field is saved to a device copy first and restored afterwards (needs that
  * much free device memory; MGP_ERR_OOM otherwise).  Results are cached per process
- * by (device, dtype, geometry, boundary kinds, operators, cycle, nsmooth, flags); set
- * MGP_TUNE_CACHE to a file name to keep them across processes.  untuned_ms / tuned_ms (either
+ * by (version of the built-in rules, device, dtype, geometry, boundary kinds, operators, cycle,
+ * nsmooth, flags); set MGP_TUNE_CACHE to a file name to keep them across processes (entries of
+ * other versions are searched again).  untuned_ms / tuned_ms (either
  * may be NULL): one iteration with the built-in choices and with the tuned ones, measured
  * after a search (0 when the cache answered). */
 int mgp_autotune(mgp_solver* s, int cycle, int64_t nsmooth, double omega, uint32_t flags, double* untuned_ms,

@@ -2496,11 +2496,17 @@ void tune_cache_load_locked() {
     }
 }
 
+// Version of the built-in launch rules, part of a configuration's key.  Values searched against
+// other rules are not taken from a file: any of them on a coarse level keeps it, and the finer
+// ones, out of the cluster, and set planes keep a level off the register form, so a file written
+// before these were built in made 33x17x17 solves slower than the built-in choices do.
+constexpr int kTuneRules = 2;
+
 std::string tune_key(const mgp_solver* s, int cycle, int64_t ns, uint32_t flags_used) {
     cudaDeviceProp p{};
     cudaGetDeviceProperties(&p, s->device);
     std::ostringstream k;
-    k << "sm" << p.major << p.minor << "x" << p.multiProcessorCount << "/" << (s->dtype == MGP_F64 ? "f64" : "f32")
+    k << "v" << kTuneRules << "/sm" << p.major << p.minor << "x" << p.multiProcessorCount << "/" << (s->dtype == MGP_F64 ? "f64" : "f32")
       << "/" << s->desc.dims[0] << "x" << s->desc.dims[1] << "x" << s->desc.dims[2] << "/L" << s->levels << "/bc";
     for (int f = 0; f < 6; f++) k << s->face_kind[f];
     k << "/r" << s->desc.relaxation << "p" << s->desc.prolongation << "q" << s->desc.restriction << "/c" << cycle
