@@ -47,11 +47,12 @@ NSMOOTH = 2
 E2E_CYCLES = 4
 REF_ARM_CYCLES = 30   # timed cycles of the reference arm (a bounded sample)
 # DRAM bytes (read + write) of one level-0 Jacobi sweep launch at this size, from an ncu capture
-# of the timed launch: ncu --set full --clock-control none --kernel-name-base demangled
+# of the timed kernel (profiles/stencil_planes_513x257x129.md): ncu --clock-control none
+#   --metrics dram__bytes_read.sum,dram__bytes_write.sum --kernel-name-base demangled
 #   -k "regex:k_stencil_planes<double, \(int\)0, \(bool\)0, \(int\)3>" -s 3 -c 1 python bench.py --kernels --steps 1
-# (289.6 MB read + 109.7 MB written; algorithmic 408.2 MB: some of u is still in L2 from the
-# launch before).
-JACOBI_SWEEP_DRAM_BYTES = 399.3e6
+# (289.6 MB read + 109.5 MB written; algorithmic 408.2 MB: the last of the result is still in L2
+# when the launch ends).
+JACOBI_SWEEP_DRAM_BYTES = 399.2e6
 CPU_BASELINE_CYCLES = 8
 NDOF = DIMS[0] * DIMS[1] * DIMS[2]
 METRIC = "F-cycle fine-grid DOF/s (FP64, 513x257x129)"

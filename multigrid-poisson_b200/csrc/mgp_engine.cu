@@ -917,7 +917,10 @@ int prolong_t(mgp_solver* s, int l) {
 // Built in only on levels of at most 2^16 points (MGP_TUNE_PROLONG_SWEEP = 2 forces it): forming
 // u' at seven points per thread makes larger levels instruction-bound -- on B200 the 513x257x129
 // F-cycle iteration took 1.585 ms fused on levels 1-4 against 1.453 ms separate, and the
-// autotuner keeps the separate passes on its 2.15M- and 277K-point levels.
+// autotuner keeps the separate passes on its 2.15M- and 277K-point levels.  Levels of at most
+// 30000 points run in the cluster, which leaves it those up to 65536 and the ones kept out; there
+// the separate passes are the faster ones by now (65^3 Jacobi F-cycle, 35937 points: 186 us per
+// iteration fused, 179 separate; 257x129x65, 36465 points: 333 and 327).
 constexpr long long kProlongSweepMaxPoints = 1ll << 16;
 bool prolong_sweep_fused(const mgp_solver* s, int l, int64_t ns) {
     const LevelState& L = s->lv[l];
@@ -1345,7 +1348,8 @@ unsigned div_magic(int d) { return d <= 1 ? 0u : (unsigned)(((1ull << 32) + d - 
 // Levels on which a sweep updates at most kClOnePoints points go to one CTA: their sweeps then end
 // with a block barrier instead of an exchange (820 cycles, more than their arithmetic).  Ten 65^3
 // red-black F-cycles 2.55 -> 2.43 ms (9^3 and 5^3 in one CTA), four 33x17x17 Jacobi ones 375 -> 363 us
-// (9x5x5); Jacobi levels of 765 and 1001 points are faster in slabs (161x97x193 by 2%).
+// (9x5x5); Jacobi levels of 765 and 1001 points are faster in slabs (161x97x193 by 2%); nothing
+// between 225 and 765 was measured for Jacobi, nor above 729 for red-black.
 constexpr long long kClOnePoints = 512;
 int slab_planes(const Geom& G, int nc, bool jacobi) {
     const int nx = G.nx;
