@@ -626,12 +626,20 @@ int short_march_chunks(const Geom& G, int bx, int cap, int chunks) {
 // keeps the march (83.9 against 85.3 us).  Longer marches on levels below that, two planes --
 // 257x129x65 FP64 sweep 14.3 -> 11.0 us, half-sweep 11.9 -> 10.4, residual 14.2 -> 12.3, FP32 sweep
 // 10.0 -> 8.7; one plane per block (the ONE form) 11.6.  Where one plane fills the chip the long
-// march stays.
+// march stays.  So it does for sweeps and the FP64 residual with its norm in long thin boxes, whose
+// plane is one block (bx == 1), part of its threads idle, and two planes per block make more
+// blocks than the chip holds (`cap`): V-cycle iteration with the sweeps in registers and as the
+// march, 4097x9x9 red-black FP64 187 and 165 us (with the norm as well 159), FP32 199 and 174,
+// Jacobi FP64 116 and 105, 2049x17x17 red-black 132 and 126; the plain residual is 1-3% apart, the
+// FP32 residual faster in registers (with norm 199 against 202).
 template <typename T, int OP>
-int planes_in_registers(const Geom& G, int ichunk, bool built_in) {
-    if (!built_in || ichunk == 1) return 0;
+int planes_in_registers(const Geom& G, int bx, int ichunk, int cap, bool norm) {
+    if (ichunk == 1) return 0;
     auto fits = [&](int P) { return (G.nx + P - 1) / P <= kMaxGridRows ? P : 0; };
-    if ((long long)G.nx * G.ny * G.nz < kShortMarchMinPoints) return fits(2);
+    if ((long long)G.nx * G.ny * G.nz < kShortMarchMinPoints) {
+        const bool sweep_or_norm64 = OP != OP_RESIDUAL || (norm && sizeof(T) == 8);
+        return bx == 1 && (G.nx + 1) / 2 > cap && sweep_or_norm64 ? 0 : fits(2);
+    }
     constexpr int kShort = sizeof(T) == 8 ? 4 : 3;
     if (ichunk > kShort || (OP == OP_RESIDUAL && sizeof(T) == 8)) return 0;
     return fits(3);
@@ -673,26 +681,24 @@ StencilShape stencil_shape(mgp_solver* s, int l, bool norm) {
     StencilShape q;
     const int plane = L.G.ny * ((L.G.nz + V - 1) / V);  // threads per plane
     q.bx = (plane + kThreads - 1) / kThreads;
-    bool built_in = true;
+    int cap = 0;  // resident blocks; 0: an explicit shape
     if constexpr (OP != OP_GS_COLUMN) {
         const bool nrm = OP == OP_RESIDUAL && norm;
         const int planes = L.tune[OP == OP_RESIDUAL ? (nrm ? MGP_TUNE_NORM_PLANES : MGP_TUNE_RESID_PLANES)
                                                     : MGP_TUNE_RELAX_PLANES];
         if (planes > 0) {
             q.chunks = (L.G.nx + planes - 1) / planes;
-            built_in = false;
         } else {
-            const int cap = sm_count(s->device) *
-                            (nrm ? (std::is_same<T, double>::value ? resident_blocks(k_residual_norm64<false>)
-                                                                    : resident_blocks(k_stencil<T, OP, true>))
-                                 : resident_blocks(k_stencil<T, OP, false>));
+            cap = sm_count(s->device) * (nrm ? (std::is_same<T, double>::value ? resident_blocks(k_residual_norm64<false>)
+                                                                               : resident_blocks(k_stencil<T, OP, true>))
+                                             : resident_blocks(k_stencil<T, OP, false>));
             q.chunks = march_chunks(q.bx, L.G.nx, cap);
             q.chunks = short_march_chunks<T>(L.G, q.bx, cap, q.chunks);
         }
     }
     q.ichunk = (L.G.nx + q.chunks - 1) / q.chunks;
     if constexpr (OP != OP_GS_COLUMN) {
-        const int P = planes_in_registers<T, OP>(L.G, q.ichunk, built_in);
+        const int P = cap ? planes_in_registers<T, OP>(L.G, q.bx, q.ichunk, cap, norm) : 0;
         q.regs = P != 0;
         if (P) q.ichunk = P;
     }
