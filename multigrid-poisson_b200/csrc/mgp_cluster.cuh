@@ -144,6 +144,9 @@ __device__ __forceinline__ bool cl_mbar_try(unsigned mb, unsigned phase) {
 }
 // The bound of a wait, and whether any CTA's wait ran out; in shared memory, read only by waits that
 // have to wait (the bound in a register cost 1.5% of the smallest solve: 33x17x17 318 -> 325 us).
+// Red-black kernels exist for the default bound too, with waits that block from their first poll:
+// the form below costs them 1-2% (65^3 FP32 F-cycles 1097 -> 1106 us, 17x25x9 414 -> 425), which
+// Jacobi gains (33x17x17 322 -> 311).
 struct ClWait {
     unsigned polls;
     int dead;
@@ -341,8 +344,16 @@ struct ClXchg {
     unsigned n, phase;
     ClWait* w;
     bool dead;  // this thread's wait ran out, or was ended by another's
+    template <bool BOUND>
     __device__ __forceinline__ bool wait(unsigned q) {
-        if (cl_mbar_wait(mb + 8 * q, (phase >> q) & 1, w)) return true;
+        if (BOUND) {
+            if (cl_mbar_wait(mb + 8 * q, (phase >> q) & 1, w)) return true;
+        } else {
+            for (unsigned n = 0; n < kWaitPolls; n++) {
+                if (cl_mbar_try(mb + 8 * q, (phase >> q) & 1)) return true;
+                if (*(const volatile int*)&w->dead) break;
+            }
+        }
         cl_raise((unsigned)__cvta_generic_to_shared(&w->dead));
         return false;
     }
@@ -456,7 +467,7 @@ __device__ __forceinline__ void cl_expect(const ClCta<T>& s, const ClXchg& X, in
 
 // Ends a sweep or residual of level L: the CTA's own values, and the neighbours' planes in its
 // halos, are there.  Every CTA calls it; those without planes of the level only count.
-template <typename T>
+template <typename T, bool BOUND>
 __device__ __forceinline__ void cl_exchange(const ClCta<T>& S, ClXchg& X) {
     const unsigned b = X.n & 1;
     X.n++;
@@ -464,11 +475,11 @@ __device__ __forceinline__ void cl_exchange(const ClCta<T>& S, ClXchg& X) {
     const bool from_left = S.la != 0u, from_right = S.ra != 0u;
     __syncthreads();
     if (from_left) {
-        if (!X.dead) X.dead = !X.wait(b);
+        if (!X.dead) X.dead = !X.wait<BOUND>(b);
         X.phase ^= 1u << b;
     }
     if (from_right) {
-        if (!X.dead) X.dead = !X.wait(2 + b);
+        if (!X.dead) X.dead = !X.wait<BOUND>(2 + b);
         X.phase ^= 4u << b;
     }
 }
@@ -492,7 +503,7 @@ __device__ __forceinline__ void cl_residual(const ClArgs<T>& a, int l, const ClC
 // Relaxation<T>::relax of level l: nsmooth Jacobi sweeps (swapping the buffers) or 2*nsmooth
 // red-black half-sweeps, the first one skipped on request.  What a thread needs for the level
 // stays in registers from sweep to sweep.
-template <typename T, bool JAC>
+template <typename T, bool JAC, bool BOUND>
 __device__ __forceinline__ void cl_relax(const ClArgs<T>& a, int l, const ClCta<T>& S, T* sm, bool skip, unsigned& cur,
                                          int& alt, ClXchg& X) {
     const ClCta<T> s = S;
@@ -525,7 +536,7 @@ __device__ __forceinline__ void cl_relax(const ClArgs<T>& a, int l, const ClCta<
                 else cl_march_pair(a, l, s, sm, src, e, lo, hi, colour, out);
             }
         }
-        cl_exchange(S, X);
+        cl_exchange<T, BOUND>(S, X);
     }
 }
 
@@ -606,7 +617,7 @@ __device__ __forceinline__ void cl_face_restrict(const ClArgs<T>& a, int l, T* s
 }
 
 // residual of level l, restriction into f_{l+1}, u_{l+1} = 0, Neumann face restriction
-template <typename T, bool JAC>
+template <typename T, bool JAC, bool BOUND>
 __device__ __forceinline__ void cl_setup(const ClArgs<T>& a, int l, T* sm, unsigned sbase, unsigned cur, int rank,
                                          const ClCta<T>* S, ClXchg& X) {
     const ClLevel<T>& F = a.L[l];
@@ -624,7 +635,7 @@ __device__ __forceinline__ void cl_setup(const ClArgs<T>& a, int l, T* sm, unsig
     };
     if (!JAC) zero_coarse();
     cl_face_restrict(a, l, sm, sbase, so_u, rank);
-    cl_exchange(S[l], X);
+    cl_exchange<T, BOUND>(S[l], X);
     // the CTA that owns fine plane 2I restricts into coarse plane I
     const int i0 = S[l].i0, np = S[l].np;
     if (np > 0) {
@@ -848,7 +859,8 @@ __device__ __forceinline__ void cl_store(const ClArgs<T>& a, const T* sm, int ra
     }
 }
 
-template <typename T, bool JAC>
+// BOUND: the waits take their bound from the arguments, else the default one.
+template <typename T, bool JAC, bool BOUND>
 __global__ void __launch_bounds__(kClMaxThreads, 1) k_cluster(const __grid_constant__ ClArgs<T> args) {
     extern __shared__ __align__(16) unsigned char cl_smem[];
     __shared__ ClArgs<T> a;
@@ -884,9 +896,9 @@ __global__ void __launch_bounds__(kClMaxThreads, 1) k_cluster(const __grid_const
     for (int q = 0; q < a.nops; q++) {
         const int l = a.lv[q], op = a.op[q];
         if (op == CL_RELAX || op == CL_RELAX_SKIP1) {
-            cl_relax<T, JAC>(a, l, S[l], sm, op == CL_RELAX_SKIP1, cur, alt, X);
+            cl_relax<T, JAC, BOUND>(a, l, S[l], sm, op == CL_RELAX_SKIP1, cur, alt, X);
         } else if (op == CL_SETUP) {
-            cl_setup<T, JAC>(a, l, sm, sbase, cur, rank, S, X);
+            cl_setup<T, JAC, BOUND>(a, l, sm, sbase, cur, rank, S, X);
         } else if (op == CL_PROLONG) {
             cl_prolong(a, l, sm, sbase, cur, rank);
             // Jacobi's next sweep only reads this CTA's u and writes the other buffer; an in-place
@@ -895,7 +907,7 @@ __global__ void __launch_bounds__(kClMaxThreads, 1) k_cluster(const __grid_const
             else cl_sync();
         } else {  // the solve loop's residual of level 0, stored, and its max-norm over the shape
             cl_residual(a, l, S[l], sm, S[l].u[(cur >> l) & 1u], X);
-            cl_exchange(S[l], X);
+            cl_exchange<T, BOUND>(S[l], X);
             const ClLevel<T>& L = a.L[l];
             const int i0 = S[l].i0, np = S[l].np;
             const Geom& G = L.G;

@@ -1317,8 +1317,9 @@ int cluster_ctas(int dev) {
     int& c = cached[dev & 63];
     if (c) return c - 1;
     int best = 0;
-    auto kernels = {(const void*)k_cluster<double, true>, (const void*)k_cluster<double, false>,
-                    (const void*)k_cluster<float, true>, (const void*)k_cluster<float, false>};
+    auto kernels = {(const void*)k_cluster<double, true, true>,   (const void*)k_cluster<float, true, true>,
+                    (const void*)k_cluster<double, false, false>, (const void*)k_cluster<float, false, false>,
+                    (const void*)k_cluster<double, false, true>,  (const void*)k_cluster<float, false, true>};
     for (int n : {16, 8}) {
         bool ok = true;
         for (const void* k : kernels) {
@@ -1564,7 +1565,9 @@ int launch_cluster(mgp_solver* s, int t, bool f, bool v, double omega, int64_t n
     cfg.stream = s->stream;
     cfg.attrs = attr;
     cfg.numAttrs = pdl_enabled() ? 2 : 1;
-    const cudaError_t e = jac ? cudaLaunchKernelEx(&cfg, k_cluster<T, true>, a) : cudaLaunchKernelEx(&cfg, k_cluster<T, false>, a);
+    const cudaError_t e = jac                        ? cudaLaunchKernelEx(&cfg, k_cluster<T, true, true>, a)
+                          : a.polls == kWaitPolls ? cudaLaunchKernelEx(&cfg, k_cluster<T, false, false>, a)
+                                                  : cudaLaunchKernelEx(&cfg, k_cluster<T, false, true>, a);
     if (e != cudaSuccess) return fail(MGP_ERR_CUDA, "kernel launch: %s", cudaGetErrorString(e));
     return check_launch(s);
 }
