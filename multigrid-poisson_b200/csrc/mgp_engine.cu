@@ -1107,7 +1107,7 @@ bool setup_residual_separate(const mgp_solver* s, int l) {
 // stream adds a branch to the captured graph at every visit, which the first solve of a solver
 // pays for (capture and instantiation), Neumann face or not; on B200, four iterations (three on
 // 257x129x65), with the side stream on every level above 30000 points, and now: 161x97x193 3.81 ->
-// 2.76 ms, 257x129x65 1.87 -> 1.33, 513x257x129 F 6.83 -> 6.17 and V 3.38 -> 3.20 (6.34 and 3.26
+// 2.74 ms, 257x129x65 1.87 -> 1.31, 513x257x129 F 6.83 -> 6.17 and V 3.38 -> 3.20 (6.34 and 3.26
 // with the limit at 2^20), 65^3 all Dirichlet 2.92 -> 2.50; later solves take the same time.
 // Above the limit the residual is a march of its own and the side stream stays.
 constexpr long long kFacesMaxPoints = kShortMarchMinPoints;
